@@ -7,7 +7,11 @@
 // points are grouped); a step is delta = K(xi) (y - X(xi)) with K the (pseudo-)inverse of J;
 // a point not yet frozen moves to xi + delta clamped to the box [-0.1, 1.1]^TD (bounds rounded
 // to f32), records |delta|_inf (the largest finite value of F when a component is not finite)
-// and freezes once that is at most the tolerance; frozen points keep xi and their last step.
+// and freezes once that is at most the tolerance; frozen points keep xi and their last step. (A
+// point's loop ends when it freezes: nothing it would still compute is kept.)
+//
+// Cells of low degree run the kernels of pullback_poly.cuh; those here take the others (pyramids,
+// intervals, degrees above 3).
 //
 // The basis at an arbitrary xi is evaluated in product form instead of the reference's
 // orthonormal expansion with a coefficient matrix (the same Lagrange functions): on intervals,
@@ -24,6 +28,7 @@
 // interleaved slots in shared memory, then each point runs its iterations. Tile layout of the
 // input points, xi and the steps as the evaluation outputs.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -33,54 +38,18 @@
 
 #include <cuda_runtime.h>
 
-#include "convert.cuh"
-#include "eval.cuh"
-#include "refcell.h"
+#include "pullback.cuh"
+#include "pullback_poly.cuh"
 #include "status.h"
 
 struct tlg_basis {
   int cell, degree, family, td;
   int64_t k;
   unsigned char* dev = nullptr;  // the basis header (tlg::BasisData)
+  tlg::PolyTerms poly = {nullptr, nullptr};  // the polynomial kernels' expansion, after the header
 };
 
 namespace tlg {
-
-constexpr int kBasisMaxN = 16;    // 1D nodes (degree + 1)
-constexpr int kBasisMaxK = 1024;  // nodes per cell
-constexpr int kPyramidMaxP = 4;   // pyramid degrees of the pull-back
-constexpr int kPyramidMaxK = 55;  // (p + 1)(p + 2)(2p + 3) / 6 at p = 4
-
-// Device copy of the basis description.
-struct alignas(16) BasisData {
-  int cell, p, k, n;        // cell type, degree, nodes per cell, 1D nodes (p + 1)
-  const double* coef;       // pyramids: C [m][k] (m-major) after this header; else null
-  double s[kBasisMaxN];     // sorted 1D nodes (tensor cells, the prism's line)
-  uint8_t idx[kBasisMaxK][4];  // per node: 1D indices (tensor) or barycentric multi-index
-                               // (simplex: lambda_0 .. lambda_TD; prism: alpha_0..2, line index)
-};
-
-struct PullBackArgs {
-  const void* nodes;
-  const uint32_t* dofmap;
-  const BasisData* basis;
-  const void* x;  // input points, GD components (absolute)
-  void* xi;       // TD components
-  void* step;     // 1 component
-  int64_t first_cell, padded, out_first_cell, x_first_cell, last_cell;
-  double origin[3];
-  double tolerance;
-  uint32_t last_node;
-  int num_points, max_iterations, tile_shift, threads;
-  int refinements;  // mixed precision: FP64-residual steps after the FP32 iteration (0: native)
-};
-
-template <typename F>
-__device__ __forceinline__ F fmax_finite();
-template <>
-__device__ __forceinline__ float fmax_finite<float>() { return 3.402823466e38f; }
-template <>
-__device__ __forceinline__ double fmax_finite<double>() { return 1.7976931348623157e308; }
 
 // 1D Lagrange values and derivatives l_i(t), l_i'(t), i < n, at the nodes s.
 template <typename F>
@@ -315,53 +284,6 @@ __device__ void map_at(const BasisData& b, const F* xs, int T, const F* xi, F* X
   }
 }
 
-// One step of a point: delta = K r, s = |delta|_inf (the largest finite value when a component
-// is not finite); a point not yet frozen moves to p + delta clamped to [lo, hi], records s and
-// freezes once s <= tol. K(t, g) at g * TD + t (in KT's precision), r and p in P's.
-template <typename P, typename KT, int TD, int GD>
-__device__ __forceinline__ void newton_update(P* p, const KT* K, const P* r, P& last, bool& frozen, P tol, P lo,
-                                              P hi, P big) {
-  P delta[TD];
-  P s = big;
-  bool bad = false;
-#pragma unroll
-  for (int t = 0; t < TD; ++t) {
-    P acc = P(K[t]) * r[0];
-#pragma unroll
-    for (int g = 1; g < GD; ++g) acc = fma(P(K[g * TD + t]), r[g], acc);
-    delta[t] = acc;
-    const P m = fabs(acc);
-    s = t == 0 ? m : (m > s ? m : s);
-    bad = bad || !(m <= big);
-  }
-  if (bad) s = big;
-  if (!frozen) {
-#pragma unroll
-    for (int d = 0; d < TD; ++d) {
-      P qd = p[d] + delta[d];
-      qd = qd < lo ? lo : qd;
-      qd = qd > hi ? hi : qd;
-      p[d] = qd;
-    }
-    last = s;
-    frozen = s <= tol;
-  }
-}
-
-// The vertex centroid of the reference cell, rounded to f32.
-__device__ __forceinline__ void centroid_f32(int cell, float* start) {
-  const float third = 1.0f / 3.0f;
-  if (cell == kTriangle) start[0] = start[1] = third;
-  else if (cell == kTetrahedron) start[0] = start[1] = start[2] = 0.25f;
-  else if (cell == kPrism) {
-    start[0] = start[1] = third;
-    start[2] = 0.5f;
-  } else if (cell == kPyramid) {
-    start[0] = start[1] = 0.4f;
-    start[2] = 0.2f;
-  } else start[0] = start[1] = start[2] = 0.5f;
-}
-
 template <typename F, int TD, int GD>
 __global__ void pull_back_kernel(const __grid_constant__ PullBackArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -411,7 +333,7 @@ __global__ void pull_back_kernel(const __grid_constant__ PullBackArgs a) {
       for (int d = 0; d < TD; ++d) p[d] = start[d];
       F last = big;
       bool frozen = false;
-      for (int it = 0; it < a.max_iterations; ++it) {
+      for (int it = 0; it < a.max_iterations && !frozen; ++it) {
         F X[GD], J[LJ], K_[LJ];
         map_at<F, TD, GD>(basis, xs, T, p, X, J);
         M::pinv(J, K_);
@@ -496,7 +418,7 @@ __global__ void pull_back_split_kernel(const __grid_constant__ PullBackArgs a) {
       for (int d = 0; d < TD; ++d) p32[d] = start[d];
       float last32 = big32;
       bool frozen32 = false;
-      for (int it = 0; it < a.max_iterations; ++it) {
+      for (int it = 0; it < a.max_iterations && !frozen32; ++it) {
         float X[GD], J[LJ], K_[LJ];
         map_at<float, TD, GD>(basis, xs32, T, p32, X, J);
         M::pinv(J, K_);
@@ -510,7 +432,7 @@ __global__ void pull_back_split_kernel(const __grid_constant__ PullBackArgs a) {
       for (int d = 0; d < TD; ++d) p[d] = f2d_exact(p32[d]);
       double last = big;
       bool frozen = false;
-      for (int it = 0; it < a.refinements; ++it) {
+      for (int it = 0; it < a.refinements && !frozen; ++it) {
         double X[GD], Jd[1];
         map_at<double, TD, GD, false>(basis, xs64, T, p, X, Jd);
         float pf[TD], X32[GD], J[LJ], K_[LJ];
@@ -533,6 +455,62 @@ __global__ void pull_back_split_kernel(const __grid_constant__ PullBackArgs a) {
 }  // namespace tlg
 
 namespace {
+
+// The expansion of the polynomial kernels: for a cell of K nodes C = V^-1 (Gauss-Jordan with
+// partial pivoting), V[j][m] = e_m(node j), e_m as in pullback_poly.cuh; checked by V C = I at the
+// nodes to 1e-12. Returns an empty vector where the kernels do not take the cell.
+std::vector<double> poly_expansion(int cell, int degree, int td, const std::vector<double>& nodes) {
+  if (degree > 3 || td < 2 || cell == tlg::kPyramid) return {};
+  const bool simplex = cell == tlg::kTriangle || cell == tlg::kTetrahedron;
+  const bool prism = cell == tlg::kPrism;
+  std::vector<std::array<int, 3>> ex;
+  for (int c = 0; c <= (td == 3 ? degree : 0); ++c)
+    for (int b = 0; b <= degree - (simplex ? c : 0); ++b)
+      for (int a = 0; a <= degree - (simplex ? b + c : prism ? b : 0); ++a) ex.push_back({a, b, c});
+  const size_t k = ex.size();
+  if (nodes.size() != k * td) return {};
+  std::vector<double> V(k * k), w(k * 2 * k, 0.0);
+  for (size_t j = 0; j < k; ++j) {
+    for (size_t m = 0; m < k; ++m) {
+      double v = 1.0;
+      for (int d = 0; d < td; ++d) {
+        const bool centred = !simplex && (!prism || d == 2);
+        const double t = nodes[j * td + d] - (centred ? 0.5 : 0.0);
+        for (int e = 0; e < ex[m][d]; ++e) v *= t;
+      }
+      V[j * k + m] = w[j * 2 * k + m] = v;
+    }
+    w[j * 2 * k + k + j] = 1.0;
+  }
+  for (size_t c = 0; c < k; ++c) {
+    size_t piv = c;
+    for (size_t r = c + 1; r < k; ++r)
+      if (std::fabs(w[r * 2 * k + c]) > std::fabs(w[piv * 2 * k + c])) piv = r;
+    if (std::fabs(w[piv * 2 * k + c]) < 1e-12) return {};
+    if (piv != c)
+      for (size_t e = 0; e < 2 * k; ++e) std::swap(w[piv * 2 * k + e], w[c * 2 * k + e]);
+    const double inv = 1.0 / w[c * 2 * k + c];
+    for (size_t e = 0; e < 2 * k; ++e) w[c * 2 * k + e] *= inv;
+    for (size_t r = 0; r < k; ++r) {
+      const double f = w[r * 2 * k + c];
+      if (r == c || f == 0.0) continue;
+      for (size_t e = 0; e < 2 * k; ++e) w[r * 2 * k + e] -= f * w[c * 2 * k + e];
+    }
+  }
+  std::vector<double> C(k * k);
+  for (size_t m = 0; m < k; ++m)
+    for (size_t i = 0; i < k; ++i) {
+      const double v = w[m * 2 * k + k + i];
+      C[m * k + i] = std::fabs(v) < 1e-13 ? 0.0 : v;
+    }
+  for (size_t j = 0; j < k; ++j)
+    for (size_t i = 0; i < k; ++i) {
+      double v = 0.0;
+      for (size_t m = 0; m < k; ++m) v += V[j * k + m] * C[m * k + i];
+      if (!(std::fabs(v - (i == j ? 1.0 : 0.0)) < 1e-12)) return {};
+    }
+  return C;
+}
 
 tlg_status basis_fail(tlg_status s, const std::string& m) { return tlg::fail(s, m); }
 
@@ -602,12 +580,31 @@ tlg_status tlg_basis_create(int cell, int degree, int family, tlg_basis** out) {
     const std::vector<double> coef =
         pyramid ? tlg::expansion_coefficients(cell, degree, family) : std::vector<double>();
     static_assert(sizeof(tlg::BasisData) % 16 == 0, "the coefficients start 16-byte aligned");
-    cudaError_t e = cudaMalloc(&b->dev, sizeof(tlg::BasisData) + coef.size() * sizeof(double));
+    // The polynomial kernels' expansion by rows, its nonzero terms only: terms, then row starts.
+    const std::vector<double> C = poly_expansion(cell, degree, td, lp);
+    std::vector<tlg::PolyTerm> terms;
+    std::vector<uint32_t> starts;
+    for (int64_t m = 0; m < k && !C.empty(); ++m) {
+      starts.push_back((uint32_t)terms.size());
+      for (int64_t i = 0; i < k; ++i)
+        if (C[m * k + i] != 0.0) terms.push_back({C[m * k + i], (int)i, 0});
+    }
+    if (!C.empty()) starts.push_back((uint32_t)terms.size());
+    const size_t off_terms = (sizeof(tlg::BasisData) + coef.size() * sizeof(double) + 15) / 16 * 16;
+    const size_t off_starts = off_terms + terms.size() * sizeof(tlg::PolyTerm);
+    cudaError_t e = cudaMalloc(&b->dev, off_starts + std::max<size_t>(starts.size(), 1) * sizeof(uint32_t));
     if (e == cudaSuccess && pyramid) h.coef = reinterpret_cast<const double*>(b->dev + sizeof(tlg::BasisData));
     if (e == cudaSuccess) e = cudaMemcpy(b->dev, &h, sizeof(h), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && pyramid)
       e = cudaMemcpy(b->dev + sizeof(tlg::BasisData), coef.data(), coef.size() * sizeof(double),
                      cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !C.empty()) {
+      b->poly.term = reinterpret_cast<const tlg::PolyTerm*>(b->dev + off_terms);
+      b->poly.start = reinterpret_cast<const uint32_t*>(b->dev + off_starts);
+      e = cudaMemcpy(b->dev + off_terms, terms.data(), terms.size() * sizeof(tlg::PolyTerm), cudaMemcpyHostToDevice);
+      if (e == cudaSuccess)
+        e = cudaMemcpy(b->dev + off_starts, starts.data(), starts.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    }
     if (e != cudaSuccess) {
       if (b->dev) cudaFree(b->dev);
       delete b;
@@ -672,6 +669,20 @@ tlg_status tlg_pull_back_block(const tlg_basis* basis, const tlg_block* b, const
   a.max_iterations = max_iterations;
   a.tile_shift = shift;
   a.refinements = refinements;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (basis->poly.term) {
+    bool found = false;
+    const cudaError_t pe =
+        refinements > 0 ? tlg::launch_pull_back_poly_split(basis->cell, basis->degree, b->gdim, a, basis->poly, s, &found)
+        : b->dtype == TLG_F64
+            ? tlg::launch_pull_back_poly_f64(basis->cell, basis->degree, b->gdim, a, basis->poly, s, &found)
+            : tlg::launch_pull_back_poly_f32(basis->cell, basis->degree, b->gdim, a, basis->poly, s, &found);
+    if (found) {
+      if (pe != cudaSuccess) return tlg::cuda_fail(pe, "tlg_pull_back_block launch");
+      tlg::record_launch(TLG_FAMILY_PULL_BACK, TLG_STRATEGY_LOOPS);
+      return tlg::ok();
+    }
+  }
   // Threads per CTA: the node slots of 128 threads, or fewer, within 96 KiB (mixed precision
   // keeps f64 and f32 copies); the basis description adds a static 4 KiB. The dynamic size is
   // always declared, as static and dynamic shared memory together may pass the default 48 KiB.
@@ -688,7 +699,6 @@ tlg_status tlg_pull_back_block(const tlg_basis* basis, const tlg_block* b, const
   const int64_t need = (a.padded + threads - 1) / threads;
   const int64_t cap = (int64_t)sms * (2048 / threads);
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min(need, cap));
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaSuccess;
 #define TLG_PB(F, TD, GD) \
   if (basis->td == TD && b->gdim == GD) { \
