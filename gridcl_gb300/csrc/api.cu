@@ -27,6 +27,8 @@
 #include "umma.cuh"
 #include "sumfact.cuh"
 #include "eval_df.cuh"
+#include "eval_poly.cuh"
+#include "poly_basis.h"
 #include "sumfact_df.cuh"
 #include "vjp.cuh"
 
@@ -98,6 +100,11 @@ struct tlg_tables {
   // the columns), copied into shared memory chunk by chunk.
   uint64_t off_umma = 0;
   int umma_kpad = 0, umma_chunks = 0;
+  // Polynomial section (f64 tables of cells of degree 1-3, eval_poly.cuh; 0 bytes elsewhere): the
+  // expansion's terms and row starts (tensor cells: the lattice's nodes in the starts), the rule's
+  // planes, lines and points; the first poly_staged bytes go to shared memory.
+  uint32_t off_poly = 0, poly_bytes = 0, poly_staged = 0, poly_starts = 0, poly_planes = 0, poly_lines = 0, poly_points = 0;
+  int poly_nplanes = 0, poly_nlines = 0;
   int* err = nullptr;
   std::vector<unsigned char> host;  // host copy of the device bytes
 };
@@ -280,9 +287,9 @@ int principal_family(uint32_t mask) {
 }
 
 // The policy of TLG_STRATEGY_AUTO for tables with sum-factorisation data, from GB300 timings of
-// curved hexahedra (ms per launch, 128^3 Q1/Q2, 64^3 Q3; paired-or-unrolled / loops / sumfact):
-// f64 Q1 4.19 / 5.00 / 3.14, Q2 34.6 / 45.3 / 13.1 (the FP64 pipe bounds, and sum factorisation
-// does a third of the multiply-adds); split Q1 0.33 / 1.21 / 0.35, Q2 1.37 / 21.9 / 1.53,
+// curved hexahedra (ms per launch, 128^3 Q1/Q2, 64^3 Q3; paired-or-unrolled / loops / sumfact): f64
+// Q3 - / 395 / 45.4 (the FP64 pipe bounds, and sum factorisation does a third of the multiply-adds;
+// Q1-Q2 and prisms P1-P2 run the polynomial kernel under either name); split Q1 0.33 / 1.21 / 0.35, Q2 1.37 / 21.9 / 1.53,
 // Q3 - / 11.5 / 0.62; f32 Q2 1.15 / 17.6 / 1.39, Q3 - / 16.7 / 0.55. So: sum factorisation
 // always in f64, and in f32 and split precision above the degrees with paired kernels
 // (quadrilaterals and hexahedra Q1-Q2).
@@ -476,6 +483,47 @@ tlg_status eval_df(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o
   if (!*found) return TLG_ERR_UNSUPPORTED;
   if (e != cudaSuccess) return cuda_fail(e, "tlg_eval_block launch");
   g_last_family = TLG_STRATEGY_DIRECT;
+  return ok();
+}
+
+// The f64 polynomial kernel; `found` is false where none is compiled for the tables (nothing
+// launched).
+tlg_status eval_poly(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o, uint32_t mask, int family,
+                     cudaStream_t stream, bool* found) {
+  *found = false;
+  if (t->poly_bytes == 0) return TLG_ERR_UNSUPPORTED;
+  tlg::PolyEvalArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.nodes = static_cast<const double*>(b->nodes);
+  a.dofmap = b->dofmap;
+  a.flags = b->flags;
+  a.tab = t->dev + t->off_poly;
+  a.refn = reinterpret_cast<const double*>(t->dev + t->off_refn);
+  void* outs[6] = {o->points, o->jacobian, o->detj, o->pinv, o->normals, o->facet_normals};
+  for (int i = 0; i < 6; ++i) a.out[i] = static_cast<double*>(outs[i]);
+  a.err = t->err;
+  a.first_cell = o->first_cell;
+  a.padded = (o->num_cells + o->tile - 1) / o->tile * o->tile;
+  a.out_first_cell = o->out_first_cell;
+  a.last_cell = b->num_cells - 1;
+  const int64_t nflags = b->flags ? std::min<int64_t>(b->num_cells, b->num_flags) : 0;
+  a.last_flag = nflags - 1;
+  for (int g = 0; g < 3; ++g) a.origin[g] = b->origin[g];
+  a.last_node = (uint32_t)(b->num_nodes - 1);
+  a.tab_bytes = t->poly_staged;
+  a.rule_global = t->poly_staged < t->poly_bytes ? 1 : 0;
+  a.off_starts = t->poly_starts;
+  a.off_planes = t->poly_planes;
+  a.off_lines = t->poly_lines;
+  a.off_points = t->poly_points;
+  a.mask = mask;
+  a.num_points = (int)t->q;
+  a.num_planes = t->poly_nplanes;
+  a.tile_shift = tile_shift(o->tile);
+  cudaError_t e = tlg::launch_eval_poly(t->cell, t->degree, t->gd, a, t->poly_nlines, stream, found);
+  if (!*found) return TLG_ERR_UNSUPPORTED;
+  if (e != cudaSuccess) return cuda_fail(e, "tlg_eval_block launch");
+  g_last_family = family;
   return ok();
 }
 
@@ -1290,7 +1338,49 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
       // Zero chunks after the last, for work items whose last group runs past it.
       host_bytes = t->off_umma + (size_t)(t->umma_chunks + tlg::kUmmaMaxGroups - 1) * 2 * tlg::kUmmaN * t->umma_kpad * 4;
     }
+    // The polynomial section.
+    std::vector<tlg::PolyTerm> pterms;
+    std::vector<uint32_t> pstarts;
+    tlg::PolyRule prule;
+    if (dtype == TLG_F64 && npoints > 0 && td >= 2 && gdim >= 2 && degree <= (cell == tlg::kTetrahedron ? 2 : 3)) {
+      const bool tensor = cell == tlg::kHexahedron || cell == tlg::kQuadrilateral;
+      if (tensor) {  // the node at each lattice position
+        std::vector<double> s1, lt;
+        if (degree <= 2 && !sf_permutation(cell, degree, family, s1, lt, pstarts)) pstarts.clear();
+      } else if (cell != tlg::kPrism || degree <= 2) {
+        const std::vector<double> C =
+            tlg::poly_expansion(cell, degree, tlg::lagrange_points(cell, degree, family), tlg::kLine);
+        for (int64_t m = 0; m < k && !C.empty(); ++m) {
+          pstarts.push_back((uint32_t)pterms.size());
+          for (int64_t i = 0; i < k; ++i)
+            if (C[m * k + i] != 0.0) pterms.push_back({C[m * k + i], (int)i, 0});
+        }
+        if (!C.empty()) pstarts.push_back((uint32_t)pterms.size());
+      }
+      if (!pstarts.empty()) {
+        prule = tlg::poly_rule(cell, degree, points, npoints);
+        t->poly_nplanes = (int)prule.planes.size();
+        t->poly_nlines = (int)prule.lines.size();
+        t->poly_starts = (uint32_t)(pterms.size() * sizeof(tlg::PolyTerm));
+        t->poly_planes = (uint32_t)align16(t->poly_starts + pstarts.size() * 4);
+        t->poly_lines = (uint32_t)(t->poly_planes + prule.planes.size() * sizeof(tlg::PolyNode));
+        t->poly_points = (uint32_t)(t->poly_lines + prule.lines.size() * sizeof(tlg::PolyNode));
+        t->poly_bytes = (uint32_t)align16(t->poly_points + prule.points.size() * sizeof(tlg::PolyNode));
+        // Rules beyond 32 KiB are read from global memory, so that they do not cost resident CTAs.
+        t->poly_staged = t->poly_bytes <= 32 * 1024 ? t->poly_bytes : t->poly_planes;
+        t->off_poly = (uint32_t)align16(host_bytes);
+        host_bytes = (size_t)t->off_poly + t->poly_bytes;
+      }
+    }
     t->host.assign(host_bytes, 0);
+    if (t->poly_bytes > 0) {
+      unsigned char* base = t->host.data() + t->off_poly;
+      if (!pterms.empty()) std::memcpy(base, pterms.data(), pterms.size() * sizeof(tlg::PolyTerm));
+      std::memcpy(base + t->poly_starts, pstarts.data(), pstarts.size() * 4);
+      std::memcpy(base + t->poly_planes, prule.planes.data(), prule.planes.size() * sizeof(tlg::PolyNode));
+      std::memcpy(base + t->poly_lines, prule.lines.data(), prule.lines.size() * sizeof(tlg::PolyNode));
+      std::memcpy(base + t->poly_points, prule.points.data(), prule.points.size() * sizeof(tlg::PolyNode));
+    }
     if (t->sf_ok) {
       std::memcpy(t->host.data() + t->off_sf, heads.data(), heads.size() * sizeof(tlg::SfBlock));
       for (size_t bi = 0; bi < sf.size(); ++bi)
@@ -1511,6 +1601,14 @@ tlg_status eval_dispatch(const tlg_tables* t, const tlg_block* b, const tlg_outp
   // A forced strategy that does not apply runs the loops kernel (strategy.rs:400-404); AUTO
   // falls through to the unrolled kernels, then the loops kernel over staged tables.
   const bool is_auto = strategy == TLG_STRATEGY_AUTO;
+  // f64 cells with a polynomial kernel: it is the sum factorisation of tensor rules (recorded so)
+  // and the direct kernel of the others.
+  if (t->poly_bytes > 0 && !t->df && (is_auto || strategy == TLG_STRATEGY_DIRECT || (strategy == TLG_STRATEGY_SUMFACT && t->sf_ok))) {
+    bool found = false;
+    const bool sf = t->sf_ok && strategy != TLG_STRATEGY_DIRECT;
+    tlg_status st = eval_poly(t, b, o, mask, sf ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT, s, &found);
+    if (found) return st;
+  }
   if (strategy == TLG_STRATEGY_SUMFACT || (is_auto && sumfact_preferred(t))) {
     bool found = false;
     tlg_status st = eval_sumfact(t, b, o, mask, s, &found);
@@ -1536,6 +1634,7 @@ tlg_status eval_dispatch(const tlg_tables* t, const tlg_block* b, const tlg_outp
   if (t->df && allow_direct) {
     bool found = false;
     tlg_status st = eval_df(t, b, o, mask, s, &found);
+    if (!found) st = eval_poly(t, b, o, mask, TLG_STRATEGY_DIRECT, s, &found);
     if (found) return st;
   }
   if (t->dtype == TLG_SPLIT32) return eval_split(t, b, o, mask, s, allow_direct, global_tables);

@@ -115,13 +115,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // default 2^22) and err[2] = 1 leaves the copy unissued, so that the wait runs out with nothing in
 // flight (the tables' test hook, tlg_tables_set_wait). Returns whether the tables arrived, the
 // same for every thread of the CTA; a CTA whose tables did not arrive computes nothing.
-__device__ __forceinline__ bool stage_table(const unsigned char* src, unsigned char* dst,
-                                            uint32_t bytes, uint64_t* bar, int* err) {
+__device__ __forceinline__ void stage_issue(const unsigned char* src, unsigned char* dst,
+                                            uint32_t bytes, uint64_t* bar, const int* err) {
   const uint32_t bar_s = (uint32_t)__cvta_generic_to_shared(bar);
   const uint32_t dst_s = (uint32_t)__cvta_generic_to_shared(dst);
-  const int limit = err ? err[1] : 0;
   const bool issue = !err || err[2] != 1;
-  const int polls = limit > 0 ? limit : (1 << 22);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_s) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -136,6 +134,13 @@ __device__ __forceinline__ bool stage_table(const unsigned char* src, unsigned c
         "l"(src), "r"(bytes), "r"(bar_s)
         : "memory");
   }
+}
+
+// Waits for stage_issue's copy; a barrier of the CTA.
+__device__ __forceinline__ bool stage_wait(uint64_t* bar, int* err) {
+  const uint32_t bar_s = (uint32_t)__cvta_generic_to_shared(bar);
+  const int limit = err ? err[1] : 0;
+  const int polls = limit > 0 ? limit : (1 << 22);
   // Bounded poll: try_wait itself suspends for a hardware-defined interval per call. On expiry
   // the error word is set and a second bounded wait gives the copy time to land (the CTA must
   // not exit with its copy in flight).
@@ -146,6 +151,12 @@ __device__ __forceinline__ bool stage_table(const unsigned char* src, unsigned c
     for (int i = 0; i < polls && !done; ++i) done = mbar_try_wait(bar_s, 0);
   }
   return __syncthreads_and(done) != 0;
+}
+
+__device__ __forceinline__ bool stage_table(const unsigned char* src, unsigned char* dst,
+                                            uint32_t bytes, uint64_t* bar, int* err) {
+  stage_issue(src, dst, bytes, bar, err);
+  return stage_wait(bar, err);
 }
 
 // ----------------------------------------------------------------------------------------

@@ -28,7 +28,6 @@
 // interleaved slots in shared memory, then each point runs its iterations. Tile layout of the
 // input points, xi and the steps as the evaluation outputs.
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -456,62 +455,6 @@ __global__ void pull_back_split_kernel(const __grid_constant__ PullBackArgs a) {
 
 namespace {
 
-// The expansion of the polynomial kernels: for a cell of K nodes C = V^-1 (Gauss-Jordan with
-// partial pivoting), V[j][m] = e_m(node j), e_m as in pullback_poly.cuh; checked by V C = I at the
-// nodes to 1e-12. Returns an empty vector where the kernels do not take the cell.
-std::vector<double> poly_expansion(int cell, int degree, int td, const std::vector<double>& nodes) {
-  if (degree > 3 || td < 2 || cell == tlg::kPyramid) return {};
-  const bool simplex = cell == tlg::kTriangle || cell == tlg::kTetrahedron;
-  const bool prism = cell == tlg::kPrism;
-  std::vector<std::array<int, 3>> ex;
-  for (int c = 0; c <= (td == 3 ? degree : 0); ++c)
-    for (int b = 0; b <= degree - (simplex ? c : 0); ++b)
-      for (int a = 0; a <= degree - (simplex ? b + c : prism ? b : 0); ++a) ex.push_back({a, b, c});
-  const size_t k = ex.size();
-  if (nodes.size() != k * td) return {};
-  std::vector<double> V(k * k), w(k * 2 * k, 0.0);
-  for (size_t j = 0; j < k; ++j) {
-    for (size_t m = 0; m < k; ++m) {
-      double v = 1.0;
-      for (int d = 0; d < td; ++d) {
-        const bool centred = !simplex && (!prism || d == 2);
-        const double t = nodes[j * td + d] - (centred ? 0.5 : 0.0);
-        for (int e = 0; e < ex[m][d]; ++e) v *= t;
-      }
-      V[j * k + m] = w[j * 2 * k + m] = v;
-    }
-    w[j * 2 * k + k + j] = 1.0;
-  }
-  for (size_t c = 0; c < k; ++c) {
-    size_t piv = c;
-    for (size_t r = c + 1; r < k; ++r)
-      if (std::fabs(w[r * 2 * k + c]) > std::fabs(w[piv * 2 * k + c])) piv = r;
-    if (std::fabs(w[piv * 2 * k + c]) < 1e-12) return {};
-    if (piv != c)
-      for (size_t e = 0; e < 2 * k; ++e) std::swap(w[piv * 2 * k + e], w[c * 2 * k + e]);
-    const double inv = 1.0 / w[c * 2 * k + c];
-    for (size_t e = 0; e < 2 * k; ++e) w[c * 2 * k + e] *= inv;
-    for (size_t r = 0; r < k; ++r) {
-      const double f = w[r * 2 * k + c];
-      if (r == c || f == 0.0) continue;
-      for (size_t e = 0; e < 2 * k; ++e) w[r * 2 * k + e] -= f * w[c * 2 * k + e];
-    }
-  }
-  std::vector<double> C(k * k);
-  for (size_t m = 0; m < k; ++m)
-    for (size_t i = 0; i < k; ++i) {
-      const double v = w[m * 2 * k + k + i];
-      C[m * k + i] = std::fabs(v) < 1e-13 ? 0.0 : v;
-    }
-  for (size_t j = 0; j < k; ++j)
-    for (size_t i = 0; i < k; ++i) {
-      double v = 0.0;
-      for (size_t m = 0; m < k; ++m) v += V[j * k + m] * C[m * k + i];
-      if (!(std::fabs(v - (i == j ? 1.0 : 0.0)) < 1e-12)) return {};
-    }
-  return C;
-}
-
 tlg_status basis_fail(tlg_status s, const std::string& m) { return tlg::fail(s, m); }
 
 }  // namespace
@@ -581,7 +524,7 @@ tlg_status tlg_basis_create(int cell, int degree, int family, tlg_basis** out) {
         pyramid ? tlg::expansion_coefficients(cell, degree, family) : std::vector<double>();
     static_assert(sizeof(tlg::BasisData) % 16 == 0, "the coefficients start 16-byte aligned");
     // The polynomial kernels' expansion by rows, its nonzero terms only: terms, then row starts.
-    const std::vector<double> C = poly_expansion(cell, degree, td, lp);
+    const std::vector<double> C = tlg::poly_expansion(cell, degree, lp, tlg::kCentred);
     std::vector<tlg::PolyTerm> terms;
     std::vector<uint32_t> starts;
     for (int64_t m = 0; m < k && !C.empty(); ++m) {

@@ -2,12 +2,14 @@
 // and the start of the iteration (pullback.cu, pullback_poly.cuh).
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 
 #include <cuda_runtime.h>
 
 #include "convert.cuh"
 #include "eval.cuh"
+#include "poly_basis.h"
 #include "refcell.h"
 
 namespace tlg {
@@ -48,15 +50,24 @@ __device__ __forceinline__ float fmax_finite<float>() { return 3.402823466e38f; 
 template <>
 __device__ __forceinline__ double fmax_finite<double>() { return 1.7976931348623157e308; }
 
+// |v| as an unsigned integer whose order is that of the magnitudes (above infinity's: NaN).
+// Comparisons of doubles take the FP64 pipe, these the integer pipes.
+__device__ __forceinline__ uint32_t magnitude(float v) { return __float_as_uint(v) & 0x7FFFFFFFu; }
+__device__ __forceinline__ unsigned long long magnitude(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+}
+__device__ __forceinline__ bool negative(float v) { return (int)__float_as_uint(v) < 0; }
+__device__ __forceinline__ bool negative(double v) { return __double2hiint(v) < 0; }
+
 // One step of a point: delta = K r, s = |delta|_inf (the largest finite value when a component
-// is not finite); a point not yet frozen moves to p + delta clamped to [lo, hi], records s and
-// freezes once s <= tol. K(t, g) at g * TD + t (in KT's precision), r and p in P's.
+// is not finite); a point not yet frozen moves to p + delta clamped to [lo, hi] (lo < 0 < hi; NaN
+// stays), records s and freezes once s <= tol (tol >= 0). K(t, g) at g * TD + t (in KT's
+// precision), r and p in P's.
 template <typename P, typename KT, int TD, int GD>
 __device__ __forceinline__ void newton_update(P* p, const KT* K, const P* r, P& last, bool& frozen, P tol, P lo,
                                               P hi, P big) {
   P delta[TD];
   P s = big;
-  bool bad = false;
 #pragma unroll
   for (int t = 0; t < TD; ++t) {
     P acc = P(K[t]) * r[0];
@@ -64,20 +75,21 @@ __device__ __forceinline__ void newton_update(P* p, const KT* K, const P* r, P& 
     for (int g = 1; g < GD; ++g) acc = fma(P(K[g * TD + t]), r[g], acc);
     delta[t] = acc;
     const P m = fabs(acc);
-    s = t == 0 ? m : (m > s ? m : s);
-    bad = bad || !(m <= big);
+    s = t == 0 || magnitude(m) > magnitude(s) ? m : s;
   }
-  if (bad) s = big;
+  if (magnitude(s) > magnitude(big)) s = big;
   if (!frozen) {
 #pragma unroll
     for (int d = 0; d < TD; ++d) {
       P qd = p[d] + delta[d];
-      qd = qd < lo ? lo : qd;
-      qd = qd > hi ? hi : qd;
+      const auto m = magnitude(qd);
+      const bool below = negative(qd);
+      const P edge = below ? lo : hi;
+      if (m > magnitude(edge) && m <= magnitude(P(INFINITY))) qd = edge;
       p[d] = qd;
     }
     last = s;
-    frozen = s <= tol;
+    frozen = magnitude(s) <= magnitude(tol);
   }
 }
 
@@ -97,7 +109,6 @@ __device__ __forceinline__ void centroid_f32(int cell, float* start) {
 
 // The polynomial kernels (pullback_poly.cuh) of f32 meshes, f64 meshes and mixed precision; `found`
 // is false where none is compiled for the cell, the degree and gdim.
-struct PolyTerms;
 cudaError_t launch_pull_back_poly_f32(int cell, int degree, int gd, const PullBackArgs& a, const PolyTerms& terms,
                                       cudaStream_t s, bool* found);
 cudaError_t launch_pull_back_poly_f64(int cell, int degree, int gd, const PullBackArgs& a, const PolyTerms& terms,

@@ -26,19 +26,10 @@
 #include <algorithm>
 
 #include "eval_launch.cuh"
+#include "poly_basis.h"
 #include "pullback.cuh"
 
 namespace tlg {
-
-// C by rows: row m's nonzero terms are term[start[m] .. start[m + 1]).
-struct PolyTerm {
-  double c;
-  int k, pad;
-};
-struct PolyTerms {
-  const uint32_t* start;
-  const PolyTerm* term;
-};
 
 struct PolyArgs {
   PullBackArgs p;

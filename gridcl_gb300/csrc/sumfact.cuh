@@ -421,9 +421,13 @@ __global__ void __launch_bounds__(kEvalThreads) sumfact_prism_kernel(const __gri
 template <typename F, bool SPLIT, bool FN>
 cudaError_t launch_sf(int td, int gd, int n, const SfArgs& a, size_t smem, cudaStream_t s, bool* found) {
   *found = true;
+  // (f64 Q1-Q2 and prisms P1-P2 run the polynomial kernel of eval_poly.cuh.)
+  constexpr bool low = sizeof(F) == 4;
   if (a.prism) {
-    if (n == 2) return launch_persistent(sumfact_prism_kernel<F, SPLIT, 2, FN>, a, a.padded, smem, s);
-    if (n == 3) return launch_persistent(sumfact_prism_kernel<F, SPLIT, 3, FN>, a, a.padded, smem, s);
+    if constexpr (low) {
+      if (n == 2) return launch_persistent(sumfact_prism_kernel<F, SPLIT, 2, FN>, a, a.padded, smem, s);
+      if (n == 3) return launch_persistent(sumfact_prism_kernel<F, SPLIT, 3, FN>, a, a.padded, smem, s);
+    }
     if (n == 4) return launch_persistent(sumfact_prism_kernel<F, SPLIT, 4, FN>, a, a.padded, smem, s);
     *found = false;
     return cudaSuccess;
@@ -431,17 +435,21 @@ cudaError_t launch_sf(int td, int gd, int n, const SfArgs& a, size_t smem, cudaS
 #define TLG_SF(TD, GD, NN) \
   if (td == TD && gd == GD && n == NN) \
     return launch_persistent(sumfact_kernel<F, SPLIT, TD, GD, NN, FN>, a, a.padded, smem, s);
-  TLG_SF(3, 3, 2)
-  TLG_SF(3, 3, 3)
+  if constexpr (low) {
+    TLG_SF(3, 3, 2)
+    TLG_SF(3, 3, 3)
+    TLG_SF(2, 2, 2)
+    TLG_SF(2, 2, 3)
+  }
   TLG_SF(3, 3, 4)
-  TLG_SF(2, 2, 2)
-  TLG_SF(2, 2, 3)
   TLG_SF(2, 2, 4)
   TLG_SF(2, 2, 5)
   TLG_SF(2, 2, 6)
   if constexpr (!FN) {  // facet normals need codimension 0
-    TLG_SF(2, 3, 2)
-    TLG_SF(2, 3, 3)
+    if constexpr (low) {
+      TLG_SF(2, 3, 2)
+      TLG_SF(2, 3, 3)
+    }
     TLG_SF(2, 3, 4)
     TLG_SF(2, 3, 5)
     TLG_SF(2, 3, 6)
