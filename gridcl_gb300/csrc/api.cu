@@ -31,6 +31,7 @@
 #include "poly_basis.h"
 #include "sumfact_df.cuh"
 #include "vjp.cuh"
+#include "vjp_poly.cuh"
 
 struct tlg_batch {
   std::vector<const tlg_tables*> tables;
@@ -101,10 +102,11 @@ struct tlg_tables {
   uint64_t off_umma = 0;
   int umma_kpad = 0, umma_chunks = 0;
   // Polynomial section (f64 tables of cells of degree 1-3, eval_poly.cuh; 0 bytes elsewhere): the
-  // expansion's terms and row starts (tensor cells: the lattice's nodes in the starts), the rule's
-  // planes, lines and points; the first poly_staged bytes go to shared memory.
-  uint32_t off_poly = 0, poly_bytes = 0, poly_staged = 0, poly_starts = 0, poly_planes = 0, poly_lines = 0, poly_points = 0;
-  int poly_nplanes = 0, poly_nlines = 0;
+  // expansion's terms and row starts (tensor cells: the lattice's nodes in the starts), the same by
+  // column, the rule's planes, lines and points; the first poly_staged bytes go to shared memory.
+  uint32_t off_poly = 0, poly_bytes = 0, poly_staged = 0, poly_starts = 0, poly_tterms = 0, poly_tstarts = 0;
+  uint32_t poly_planes = 0, poly_lines = 0, poly_points = 0;
+  int poly_nplanes = 0, poly_nlines = 0, poly_plane_lines = 0;  // (the most lines of a plane)
   int* err = nullptr;
   std::vector<unsigned char> host;  // host copy of the device bytes
 };
@@ -486,6 +488,20 @@ tlg_status eval_df(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o
   return ok();
 }
 
+tlg::PolyCells poly_cells(const tlg_tables* t, const tlg_block* b, int64_t first_cell) {
+  tlg::PolyCells c;
+  c.nodes = static_cast<const double*>(b->nodes);
+  c.dofmap = b->dofmap;
+  c.tab = t->dev + t->off_poly;
+  c.err = t->err;
+  c.first_cell = first_cell;
+  c.last_cell = b->num_cells - 1;
+  c.last_node = (uint32_t)(b->num_nodes - 1);
+  c.tab_bytes = t->poly_staged;
+  c.off_starts = t->poly_starts;
+  return c;
+}
+
 // The f64 polynomial kernel; `found` is false where none is compiled for the tables (nothing
 // launched).
 tlg_status eval_poly(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o, uint32_t mask, int family,
@@ -494,25 +510,17 @@ tlg_status eval_poly(const tlg_tables* t, const tlg_block* b, const tlg_outputs*
   if (t->poly_bytes == 0) return TLG_ERR_UNSUPPORTED;
   tlg::PolyEvalArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.nodes = static_cast<const double*>(b->nodes);
-  a.dofmap = b->dofmap;
+  a.cells = poly_cells(t, b, o->first_cell);
   a.flags = b->flags;
-  a.tab = t->dev + t->off_poly;
   a.refn = reinterpret_cast<const double*>(t->dev + t->off_refn);
   void* outs[6] = {o->points, o->jacobian, o->detj, o->pinv, o->normals, o->facet_normals};
   for (int i = 0; i < 6; ++i) a.out[i] = static_cast<double*>(outs[i]);
-  a.err = t->err;
-  a.first_cell = o->first_cell;
   a.padded = (o->num_cells + o->tile - 1) / o->tile * o->tile;
   a.out_first_cell = o->out_first_cell;
-  a.last_cell = b->num_cells - 1;
   const int64_t nflags = b->flags ? std::min<int64_t>(b->num_cells, b->num_flags) : 0;
   a.last_flag = nflags - 1;
   for (int g = 0; g < 3; ++g) a.origin[g] = b->origin[g];
-  a.last_node = (uint32_t)(b->num_nodes - 1);
-  a.tab_bytes = t->poly_staged;
   a.rule_global = t->poly_staged < t->poly_bytes ? 1 : 0;
-  a.off_starts = t->poly_starts;
   a.off_planes = t->poly_planes;
   a.off_lines = t->poly_lines;
   a.off_points = t->poly_points;
@@ -1342,7 +1350,7 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
     std::vector<tlg::PolyTerm> pterms;
     std::vector<uint32_t> pstarts;
     tlg::PolyRule prule;
-    if (dtype == TLG_F64 && npoints > 0 && td >= 2 && gdim >= 2 && degree <= (cell == tlg::kTetrahedron ? 2 : 3)) {
+    if (dtype == TLG_F64 && npoints > 0 && td >= 2 && gdim >= 2 && degree <= 3) {
       const bool tensor = cell == tlg::kHexahedron || cell == tlg::kQuadrilateral;
       if (tensor) {  // the node at each lattice position
         std::vector<double> s1, lt;
@@ -1361,8 +1369,11 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
         prule = tlg::poly_rule(cell, degree, points, npoints);
         t->poly_nplanes = (int)prule.planes.size();
         t->poly_nlines = (int)prule.lines.size();
+        for (const tlg::PolyNode& p : prule.planes) t->poly_plane_lines = std::max(t->poly_plane_lines, p.count);
         t->poly_starts = (uint32_t)(pterms.size() * sizeof(tlg::PolyTerm));
-        t->poly_planes = (uint32_t)align16(t->poly_starts + pstarts.size() * 4);
+        t->poly_tterms = (uint32_t)align16(t->poly_starts + pstarts.size() * 4);
+        t->poly_tstarts = (uint32_t)(t->poly_tterms + pterms.size() * sizeof(tlg::PolyTerm));
+        t->poly_planes = (uint32_t)align16(t->poly_tstarts + (tensor ? 0 : (size_t)k + 1) * 4);
         t->poly_lines = (uint32_t)(t->poly_planes + prule.planes.size() * sizeof(tlg::PolyNode));
         t->poly_points = (uint32_t)(t->poly_lines + prule.lines.size() * sizeof(tlg::PolyNode));
         t->poly_bytes = (uint32_t)align16(t->poly_points + prule.points.size() * sizeof(tlg::PolyNode));
@@ -1377,6 +1388,19 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
       unsigned char* base = t->host.data() + t->off_poly;
       if (!pterms.empty()) std::memcpy(base, pterms.data(), pterms.size() * sizeof(tlg::PolyTerm));
       std::memcpy(base + t->poly_starts, pstarts.data(), pstarts.size() * 4);
+      if (!pterms.empty()) {  // by column: node k's (coefficient, m), m ascending
+        std::vector<tlg::PolyTerm> cols;
+        std::vector<uint32_t> cstarts;
+        for (int64_t i = 0; i < k; ++i) {
+          cstarts.push_back((uint32_t)cols.size());
+          for (int64_t m = 0; m < k; ++m)
+            for (uint32_t e = pstarts[m]; e < pstarts[m + 1]; ++e)
+              if (pterms[e].k == (int)i) cols.push_back({pterms[e].c, (int)m, 0});
+        }
+        cstarts.push_back((uint32_t)cols.size());
+        std::memcpy(base + t->poly_tterms, cols.data(), cols.size() * sizeof(tlg::PolyTerm));
+        std::memcpy(base + t->poly_tstarts, cstarts.data(), cstarts.size() * 4);
+      }
       std::memcpy(base + t->poly_planes, prule.planes.data(), prule.planes.size() * sizeof(tlg::PolyNode));
       std::memcpy(base + t->poly_lines, prule.lines.data(), prule.lines.size() * sizeof(tlg::PolyNode));
       std::memcpy(base + t->poly_points, prule.points.data(), prule.points.size() * sizeof(tlg::PolyNode));
@@ -1816,6 +1840,38 @@ tlg_status vjp_sumfact(const tlg_tables* t, const tlg::VjpArgs& v, cudaStream_t 
   return ok();
 }
 
+// The f64 polynomial adjoint from the arguments of the node-row kernel; `found` is false where none
+// is compiled for the tables.
+tlg_status vjp_poly(const tlg_tables* t, const tlg_block* b, const tlg::VjpArgs& v, int family, cudaStream_t s,
+                    bool* found) {
+  *found = false;
+  if (t->poly_bytes == 0 || t->td != t->gd) return TLG_ERR_UNSUPPORTED;
+  tlg::VjpPolyArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.cells = poly_cells(t, b, v.first_cell);
+  for (int i = 0; i < 3; ++i) a.ct[i] = static_cast<const double*>(v.ct[i]);
+  for (int i = 0; i < 4; ++i) a.out[i] = static_cast<double*>(v.out[i]);
+  a.local = static_cast<double*>(v.local);
+  a.padded = v.padded;
+  a.out_first_cell = v.out_first_cell;
+  a.range_end = v.range_end;
+  for (int g = 0; g < 3; ++g) a.origin[g] = v.origin[g];
+  a.off_planes = t->poly_planes;
+  a.off_lines = t->poly_lines;
+  a.off_points = t->poly_points;
+  a.off_tterms = t->poly_tterms;
+  a.off_tstarts = t->poly_tstarts;
+  a.num_points = v.num_points;
+  a.num_planes = t->poly_nplanes;
+  a.plane_lines = t->poly_plane_lines;
+  a.rule_global = t->poly_staged < t->poly_bytes ? 1 : 0;
+  cudaError_t e = tlg::launch_vjp_poly(t->cell, t->degree, a, t->poly_nlines, s, found);
+  if (!*found) return TLG_ERR_UNSUPPORTED;
+  if (e != cudaSuccess) return cuda_fail(e, "tlg_vjp_block launch");
+  g_last_family = family;
+  return ok();
+}
+
 // The sum-factorised adjoint from forward fields already written (det J and K in o->detj and
 // o->pinv, read); `found` is false where it does not apply.
 tlg_status vjp_sumfact_from_fields(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o,
@@ -2019,6 +2075,13 @@ tlg_status tlg_vjp_block(const tlg_tables* t, const tlg_block* b, const tlg_outp
   const size_t smem = (t->vjp_bytes + 15) / 16 * 16 + tlg::vjp_stage_bytes(split, t->td, (int)t->k);
   bool found = false;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const bool sumfact = strategy == TLG_STRATEGY_SUMFACT || strategy == TLG_STRATEGY_AUTO;
+  // f64 cells with a polynomial kernel: it takes the place of both.
+  if (t->poly_bytes > 0) {
+    const int family = sumfact && vjp_sumfact_preferred(t) ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT;
+    tlg_status st = vjp_poly(t, b, a, family, s, &found);
+    if (found) return st;
+  }
   if (strategy == TLG_STRATEGY_SUMFACT || (strategy == TLG_STRATEGY_AUTO && vjp_sumfact_preferred(t))) {
     tlg_status st = vjp_sumfact(t, a, s, &found);
     if (found) return st;

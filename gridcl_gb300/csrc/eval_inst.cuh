@@ -1,6 +1,6 @@
 // Instantiation list of the scalar evaluation kernels for one scalar type (included by
 // eval_f32.cu and eval_f64.cu with TLG_F and TLG_LAUNCH defined). Unrolled direct kernels exist
-// for f64 at P3 tetrahedra, pyramids, P4 triangles and intervals (other f64 cells of low degree run the polynomial
+// for f64 at pyramids, P4 triangles and intervals (other f64 cells of low degree run the polynomial
 // kernel of eval_poly.cuh, f32 at tile 16 the paired kernel of eval_pair.cu); every other (TD, GD, K,
 // tile) runs the loops kernel.
 #include "eval_launch.cuh"
@@ -16,8 +16,7 @@ cudaError_t TLG_LAUNCH(int td, int gd, int k, const EvalArgs<TLG_F>& a, size_t s
 #define TLG_DIRECT(TD, GD, K) \
   if (*direct && td == TD && gd == GD && k == K) \
     return launch_persistent(eval_direct_kernel<TLG_F, TD, GD, K, 16>, a, a.padded, smem, s);
-  // Tetrahedra P3, pyramids P1-P3.
-  TLG_DIRECT(3, 3, 20)
+  // Pyramids P1-P3.
   TLG_DIRECT(3, 3, 5)
   TLG_DIRECT(3, 3, 14)
   TLG_DIRECT(3, 3, 30)

@@ -10,6 +10,7 @@ cudaError_t launch_eval_poly(int cell, int degree, int gd, const PolyEvalArgs& a
   if (cell == CELL && degree == P && gd == GD) return launch_poly_cell<CELL, P, GD>(a, lines, s);
   TLG_X(kTetrahedron, 1, 3)
   TLG_X(kTetrahedron, 2, 3)
+  TLG_X(kTetrahedron, 3, 3)
   TLG_X(kHexahedron, 1, 3)
   TLG_X(kHexahedron, 2, 3)
   TLG_X(kPrism, 1, 3)

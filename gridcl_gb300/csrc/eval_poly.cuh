@@ -1,5 +1,5 @@
 // f64 evaluation on the polynomial form of a cell's map, line by line of its point set: tetrahedra
-// P1-P2, triangles P1-P3, hexahedra and quadrilaterals Q1-Q2, prisms P1-P2, facet rules included.
+// and triangles P1-P3, hexahedra and quadrilaterals Q1-Q2, prisms P1-P2, facet rules included.
 //
 // GB300's FP64 pipe does one multiply-add per 16 cycles and SM for a whole warp, so the f64 fields
 // cost what their FP64 operations cost. The map of a cell is x_0 + sum_abc c_abc e_a(x) e_b(y) e_c(z)
@@ -42,17 +42,25 @@
 
 namespace tlg {
 
-struct PolyEvalArgs {
+// The mesh's and the table's side of a launch. tab: PolyTerm terms by row and row starts, the same
+// by column, PolyNode planes, lines, points (poly_basis.h); its first tab_bytes are staged.
+struct PolyCells {
   const double* nodes;
   const uint32_t* dofmap;
-  const uint32_t* flags;
-  const unsigned char* tab;  // PolyTerm terms, row starts, PolyNode planes, lines, points (poly_basis.h)
-  const double* refn;        // [Q][TD] reference normals (facet rules)
-  double* out[6];
+  const unsigned char* tab;
   int* err;
-  int64_t first_cell, padded, out_first_cell, last_cell, last_flag;
+  int64_t first_cell, last_cell;
+  uint32_t last_node, tab_bytes, off_starts;
+};
+
+struct PolyEvalArgs {
+  PolyCells cells;
+  const uint32_t* flags;
+  const double* refn;  // [Q][TD] reference normals (facet rules)
+  double* out[6];
+  int64_t padded, out_first_cell, last_flag;
   double origin[3];
-  uint32_t last_node, tab_bytes, off_starts, off_planes, off_lines, off_points, mask;  // tab_bytes: staged
+  uint32_t off_planes, off_lines, off_points, mask;
   int num_points, num_planes, tile_shift;
   int rule_global;  // only the terms and row starts are staged, the rule is read from global memory
   int batch;  // planes whose sums are held at a time
@@ -65,6 +73,7 @@ struct PolySpace {
   static constexpr int TD = CELL == kTriangle || CELL == kQuadrilateral ? 2 : 3;
   static constexpr bool kTri = CELL == kTriangle || CELL == kTetrahedron || CELL == kPrism;  // simplex in (x, y)
   static constexpr bool kTet = CELL == kTetrahedron;
+  static constexpr bool kTensor = CELL == kHexahedron || CELL == kQuadrilateral;
   static constexpr int N = P + 1;
   static constexpr int AB = kTri ? N * (N + 1) / 2 : N * N;         // P_ab
   static constexpr int QAB = kTet ? P * (P + 1) / 2 : AB;           // Q_ab
@@ -199,31 +208,19 @@ __device__ __forceinline__ void poly_point(const PolyAt& x, bool want_x, bool wa
   }
 }
 
-// W: cells of a CTA, 16 or 32.
+// The CTA's cells c0 .. c0 + W - 1: the rule and expansion staged (stage_issue's copy, begun here),
+// the nodes, and the coefficients c_abc in cs [K][GD][W] (tensor cells: ys itself). Returns whether
+// the table arrived; a barrier of the CTA.
 template <int CELL, int P, int GD, int W>
-__global__ void __launch_bounds__(W == 32 ? 288 : 192, 2) eval_poly_kernel(const __grid_constant__ PolyEvalArgs a) {
+__device__ __forceinline__ bool poly_coefficients(const PolyCells& a, int64_t c0, unsigned char* smem, uint64_t* bar,
+                                                  double* ys, double* cs) {
   using S = PolySpace<CELL, P>;
   constexpr int TD = S::TD, K = S::K, N = S::N;
-  constexpr bool MID = !S::kTri && P == 2;  // x, y about the centre
-  constexpr bool MIDZ = !S::kTet && P == 2;
-  constexpr bool TENSOR = CELL == kHexahedron || CELL == kQuadrilateral;
-  constexpr bool AFFINE = S::kTri && TD == (S::kTet ? 3 : 2) && P == 1;
-  constexpr int REF = TENSOR && N == 3 ? K / 2 : 0;  // lattice position of the constant's node
-  using M = Factors<double, TD, GD>;
-  __shared__ uint64_t bar;
-  extern __shared__ __align__(16) unsigned char smem[];
-  stage_issue(a.tab, smem, a.tab_bytes, &bar, a.err);
-  double* ys = reinterpret_cast<double*>(smem + a.tab_bytes);  // [K][GD][W]: nodes, tensor cells in place
-  double* cs = TENSOR ? ys : ys + K * GD * W;                  // coefficients
-  double* pl = cs + K * GD * W;                                // [batch][PLANE][GD][W]
-  const unsigned char* rule = a.rule_global ? a.tab : smem;
-  const PolyNode* planes = reinterpret_cast<const PolyNode*>(rule + a.off_planes);
-  const PolyNode* lines = reinterpret_cast<const PolyNode*>(rule + a.off_lines);
-  const PolyNode* points = reinterpret_cast<const PolyNode*>(rule + a.off_points);
+  constexpr bool TENSOR = S::kTensor;
+  stage_issue(a.tab, smem, a.tab_bytes, bar, a.err);
   const PolyTerm* terms = reinterpret_cast<const PolyTerm*>(smem);
   const uint32_t* starts = reinterpret_cast<const uint32_t*>(smem + a.off_starts);
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int64_t c0 = (int64_t)blockIdx.x * W;
   // The nodes, while the table is on its way: x_k - x_0 at k (tensor cells: x_k).
   for (int i = tid; i < K * W; i += nt) {
     const int lane = i % W, k = i / W;
@@ -235,7 +232,7 @@ __global__ void __launch_bounds__(W == 32 ? 288 : 192, 2) eval_poly_kernel(const
       ys[(k * GD + g) * W + lane] = TENSOR ? v : __dsub_rn(v, __ldg(a.nodes + n0 * GD + g));
     }
   }
-  if (!stage_wait(&bar, a.err)) return;  // (a barrier of the CTA)
+  if (!stage_wait(bar, a.err)) return false;
   if constexpr (TENSOR) {
     // Lattice order first (node starts[m] at lattice position m), one (g, cell) per thread; then
     // a direction at a time, in place: (u_0, u_1) -> (u_0, u_1 - u_0) or (u_0, u_1, u_2) -> (u_1,
@@ -291,6 +288,60 @@ __global__ void __launch_bounds__(W == 32 ? 288 : 192, 2) eval_poly_kernel(const
   }
   __syncthreads();
 
+  return true;
+}
+
+// det J and, with want_k, K of a volume cell's J (codimension 0): K's rows by cofactors (K(t, g) at
+// TD g + t), det J by the first column's, which are row 0 of K.
+template <int D>
+__device__ __forceinline__ void poly_square(const double* j, bool want_k, double& dj, double* kk) {
+  using M = Factors<double, D, D>;
+  if constexpr (D == 3) {
+    kk[0] = M::cross(j[4], j[8], j[7], j[5]);
+    kk[3] = M::cross(j[6], j[5], j[3], j[8]);
+    kk[6] = M::cross(j[3], j[7], j[6], j[4]);
+    dj = fma(j[2], kk[6], fma(j[1], kk[3], __dmul_rn(j[0], kk[0])));
+    if (want_k) {
+      kk[1] = M::cross(j[7], j[2], j[1], j[8]);
+      kk[4] = M::cross(j[0], j[8], j[6], j[2]);
+      kk[7] = M::cross(j[6], j[1], j[0], j[7]);
+      kk[2] = M::cross(j[1], j[5], j[4], j[2]);
+      kk[5] = M::cross(j[3], j[2], j[0], j[5]);
+      kk[8] = M::cross(j[0], j[4], j[3], j[1]);
+      const double inv = __drcp_rn(dj);
+#pragma unroll
+      for (int r = 0; r < 9; ++r) kk[r] = __dmul_rn(kk[r], inv);
+    }
+  } else {
+    dj = M::detj(j);
+    if (want_k) M::pinv(j, kk);
+  }
+}
+
+// W: cells of a CTA, 16 or 32.
+template <int CELL, int P, int GD, int W>
+__global__ void __launch_bounds__(W == 32 ? 288 : 192, 2) eval_poly_kernel(const __grid_constant__ PolyEvalArgs a) {
+  using S = PolySpace<CELL, P>;
+  constexpr int TD = S::TD, K = S::K, N = S::N;
+  constexpr bool MID = !S::kTri && P == 2;  // x, y about the centre
+  constexpr bool MIDZ = !S::kTet && P == 2;
+  constexpr bool TENSOR = S::kTensor;
+  constexpr bool AFFINE = S::kTri && TD == (S::kTet ? 3 : 2) && P == 1;
+  constexpr int REF = TENSOR && N == 3 ? K / 2 : 0;  // lattice position of the constant's node
+  using M = Factors<double, TD, GD>;
+  __shared__ uint64_t bar;
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* ys = reinterpret_cast<double*>(smem + a.cells.tab_bytes);  // [K][GD][W]: nodes, tensor cells in place
+  double* cs = TENSOR ? ys : ys + K * GD * W;                  // coefficients
+  double* pl = cs + K * GD * W;                                // [batch][PLANE][GD][W]
+  const unsigned char* rule = a.rule_global ? a.cells.tab : smem;
+  const PolyNode* planes = reinterpret_cast<const PolyNode*>(rule + a.off_planes);
+  const PolyNode* lines = reinterpret_cast<const PolyNode*>(rule + a.off_lines);
+  const PolyNode* points = reinterpret_cast<const PolyNode*>(rule + a.off_points);
+  const uint32_t* starts = reinterpret_cast<const uint32_t*>(smem + a.cells.off_starts);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int64_t c0 = (int64_t)blockIdx.x * W;
+  if (!poly_coefficients<CELL, P, GD, W>(a.cells, c0, smem, &bar, ys, cs)) return;
   const uint32_t mask = a.mask;
   const bool want_x = (mask & kOutPoints) != 0, want_j = (mask & ~kOutPoints) != 0;
   const bool want_k = (mask & (kOutPinv | kOutFacetNormals)) != 0;
@@ -321,14 +372,14 @@ __global__ void __launch_bounds__(W == 32 ? 288 : 192, 2) eval_poly_kernel(const
       double A[GD][N], D[GD][S::DA + 1], E[GD][S::EA + 1];
       if (MID && y.mid) poly_line<CELL, P, GD, W, MID>(sums, y, want_j, A, D, E);
       else poly_line<CELL, P, GD, W, false>(sums, y, want_j, A, D, E);
-      const uint32_t* row = a.dofmap + min(a.first_cell + c, a.last_cell) * K;
-      const int64_t n0 = min(__ldg(row + (TENSOR ? starts[REF] : 0)), a.last_node);
+      const uint32_t* row = a.cells.dofmap + min(a.cells.first_cell + c, a.cells.last_cell) * K;
+      const int64_t n0 = min(__ldg(row + (TENSOR ? starts[REF] : 0)), a.cells.last_node);
       double xo[GD];
 #pragma unroll
-      for (int g = 0; g < GD; ++g) xo[g] = __dadd_rn(__ldg(a.nodes + n0 * GD + g), a.origin[g]);
+      for (int g = 0; g < GD; ++g) xo[g] = __dadd_rn(__ldg(a.cells.nodes + n0 * GD + g), a.origin[g]);
       double sign = 1.0;
       if ((mask & kOutNormals) && a.flags != nullptr && a.last_flag >= 0)
-        sign = (__ldg(a.flags + min(a.first_cell + c, a.last_flag)) & 1u) ? -1.0 : 1.0;
+        sign = (__ldg(a.flags + min(a.cells.first_cell + c, a.last_flag)) & 1u) ? -1.0 : 1.0;
       const int64_t o = a.out_first_cell + c;
       const int64_t tile = o >> a.tile_shift;
       const int ol = (int)(o & tmask);
@@ -348,24 +399,9 @@ __global__ void __launch_bounds__(W == 32 ? 288 : 192, 2) eval_poly_kernel(const
         }
         if (!want_j) continue;
         if (new_j) {
-          if constexpr (TD == 3) {
-            // K's rows by cofactors (K(t, g) at 3 g + t); row 0 = J_1 x J_2 gives det J.
-            kk[0] = M::cross(j[4], j[8], j[7], j[5]);
-            kk[3] = M::cross(j[6], j[5], j[3], j[8]);
-            kk[6] = M::cross(j[3], j[7], j[6], j[4]);
-            dj = fma(j[2], kk[6], fma(j[1], kk[3], __dmul_rn(j[0], kk[0])));
-            if (want_k) {
-              kk[1] = M::cross(j[7], j[2], j[1], j[8]);
-              kk[4] = M::cross(j[0], j[8], j[6], j[2]);
-              kk[7] = M::cross(j[6], j[1], j[0], j[7]);
-              kk[2] = M::cross(j[1], j[5], j[4], j[2]);
-              kk[5] = M::cross(j[3], j[2], j[0], j[5]);
-              kk[8] = M::cross(j[0], j[4], j[3], j[1]);
-              const double inv = __drcp_rn(dj);
-#pragma unroll
-              for (int r = 0; r < 9; ++r) kk[r] = __dmul_rn(kk[r], inv);
-            }
-          } else if constexpr (GD == 3) {
+          if constexpr (TD == GD) {
+            poly_square<TD>(j, want_k, dj, kk);
+          } else {
             // One cross product and length for the area element and the normal (the operations
             // of Factors::detj and Factors::normal).
             if (mask & (kOutDetJ | kOutNormals)) {
@@ -376,9 +412,6 @@ __global__ void __launch_bounds__(W == 32 ? 288 : 192, 2) eval_poly_kernel(const
 #pragma unroll
                 for (int g = 0; g < 3; ++g) nrm[g] = __ddiv_rn(__dmul_rn(sign, v[g]), dj);
             }
-            if (want_k) M::pinv(j, kk);
-          } else {
-            if (mask & kOutDetJ) dj = M::detj(j);
             if (want_k) M::pinv(j, kk);
           }
         }
@@ -434,7 +467,7 @@ inline cudaError_t launch_poly_width(PolyEvalArgs a, int lines, cudaStream_t s) 
   auto kern = eval_poly_kernel<CELL, P, GD, W>;
   a.batch = poly_batch<CELL, P, GD>(a.num_planes);
   const size_t value_bytes = (size_t)GD * W * 8;
-  const size_t smem = a.tab_bytes + (size_t)(tensor ? 1 : 2) * S::K * value_bytes +
+  const size_t smem = a.cells.tab_bytes + (size_t)(tensor ? 1 : 2) * S::K * value_bytes +
                       (S::TD == 3 ? (size_t)a.batch * S::PLANE * value_bytes : 0);
   cudaError_t e = cudaSuccess;
   if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -445,6 +478,17 @@ inline cudaError_t launch_poly_width(PolyEvalArgs a, int lines, cudaStream_t s) 
   return cudaGetLastError();
 }
 
+// SMs of the device, queried once per thread.
+inline int poly_sms() {
+  static thread_local int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return sms;
+}
+
 // Cells of a CTA: 16; 32 for the cells whose kernels leave out a middle point's terms (tensor
 // directions at degree 2), so that a warp is one line and its lanes agree on the branch, once the
 // 32-cell CTAs fill the SMs twice (Q2 hexahedra at 27 points, ms with 32 / 16 cells: 226,981 cells
@@ -452,13 +496,7 @@ inline cudaError_t launch_poly_width(PolyEvalArgs a, int lines, cudaStream_t s) 
 template <int CELL, int P, int GD>
 inline cudaError_t launch_poly_cell(const PolyEvalArgs& a, int lines, cudaStream_t s) {
   if constexpr (P == 2 && (CELL == kHexahedron || CELL == kPrism || CELL == kQuadrilateral)) {
-    static thread_local int sms = 0;
-    if (sms == 0) {
-      int dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
-    if (a.padded >= (int64_t)64 * sms) return launch_poly_width<CELL, P, GD, 32>(a, lines, s);
+    if (a.padded >= (int64_t)64 * poly_sms()) return launch_poly_width<CELL, P, GD, 32>(a, lines, s);
   }
   return launch_poly_width<CELL, P, GD, 16>(a, lines, s);
 }

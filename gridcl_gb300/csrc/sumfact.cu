@@ -8,6 +8,7 @@
 namespace tlg {
 
 
+// (f64 runs the polynomial kernel of vjp_poly.cuh.)
 cudaError_t launch_vjp_sumfact(bool split, int n, const VjpSfArgs& a, size_t smem, int threads, cudaStream_t s,
                                bool* found) {
   *found = true;
@@ -29,9 +30,6 @@ cudaError_t launch_vjp_sumfact(bool split, int n, const VjpSfArgs& a, size_t sme
   if (split) {
     TLG_VSF(float, true, 2)
     TLG_VSF(float, true, 3)
-  } else {
-    TLG_VSF(double, false, 2)
-    TLG_VSF(double, false, 3)
   }
 #undef TLG_VSF
   *found = false;
