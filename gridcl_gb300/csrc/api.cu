@@ -27,6 +27,7 @@
 #include "umma.cuh"
 #include "sumfact.cuh"
 #include "eval_df.cuh"
+#include "eval_dfpoly.cuh"
 #include "eval_poly.cuh"
 #include "poly_basis.h"
 #include "sumfact_df.cuh"
@@ -107,6 +108,8 @@ struct tlg_tables {
   uint32_t off_poly = 0, poly_bytes = 0, poly_staged = 0, poly_starts = 0, poly_tterms = 0, poly_tstarts = 0;
   uint32_t poly_planes = 0, poly_lines = 0, poly_points = 0;
   int poly_nplanes = 0, poly_nlines = 0, poly_plane_lines = 0;  // (the most lines of a plane)
+  // Double-float tables: the rule's lines and points as PolyDfNode.
+  uint32_t off_polydf = 0, polydf_bytes = 0, polydf_points = 0;
   int* err = nullptr;
   std::vector<unsigned char> host;  // host copy of the device bytes
 };
@@ -529,6 +532,45 @@ tlg_status eval_poly(const tlg_tables* t, const tlg_block* b, const tlg_outputs*
   a.num_planes = t->poly_nplanes;
   a.tile_shift = tile_shift(o->tile);
   cudaError_t e = tlg::launch_eval_poly(t->cell, t->degree, t->gd, a, t->poly_nlines, stream, found);
+  if (!*found) return TLG_ERR_UNSUPPORTED;
+  if (e != cudaSuccess) return cuda_fail(e, "tlg_eval_block launch");
+  g_last_family = family;
+  return ok();
+}
+
+// The double-float polynomial kernel (TLG_DF64 tables of volume cells, tile 16, no facet normals);
+// `found` is false where none is compiled for the tables.
+tlg_status eval_dfpoly(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o, uint32_t mask, int family,
+                       cudaStream_t stream, bool* found) {
+  *found = false;
+  if (t->polydf_bytes == 0 || o->tile != 16 || (mask & tlg::kOutFacetNormals)) return TLG_ERR_UNSUPPORTED;
+  // Prisms with one line per plane (a triangle rule of distinct y, or of one row): the prism kernel, whose
+  // triangle stage serves every z, is the faster (GB300, ms, this kernel / that one: P2, 300,000 cells, 3 x 1
+  // x 7 points 1.18 / 0.59, 3 x 3 x 3 points 0.78 / 0.96; P1, 500,000 cells, 3 x 1 x 2 0.28 / 0.26, 2 x 2 x 2
+  // 0.29 / 0.33).
+  if (t->cell == tlg::kPrism && t->sf_ok && t->poly_plane_lines < 2) return TLG_ERR_UNSUPPORTED;
+  tlg::PolyDfArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.cells = poly_cells(t, b, o->first_cell);
+  a.dftab = t->dev + t->off_polydf;
+  a.dftab_bytes = t->polydf_bytes <= 24 * 1024 ? t->polydf_bytes : 0;
+  void* outs[4] = {o->points, o->jacobian, o->detj, o->pinv};
+  a.wide = 1;
+  for (int i = 0; i < 4; ++i) {
+    a.out[i] = static_cast<double*>(outs[i]);
+    if (reinterpret_cast<uintptr_t>(outs[i]) % 16 != 0) a.wide = 0;
+  }
+  a.padded = (o->num_cells + 15) / 16 * 16;
+  a.out_first_cell = o->out_first_cell;
+  for (int g = 0; g < 3; ++g) a.origin[g] = b->origin[g];
+  a.off_planes = t->poly_planes;
+  a.off_dfpoints = t->polydf_points;
+  a.mask = mask;
+  a.num_points = (int)t->q;
+  a.num_planes = t->poly_nplanes;
+  a.plane_lines = t->poly_plane_lines;
+  a.rule_global = t->poly_staged < t->poly_bytes ? 1 : 0;
+  cudaError_t e = tlg::launch_eval_dfpoly(t->cell, t->degree, a, t->poly_nlines, stream, found);
   if (!*found) return TLG_ERR_UNSUPPORTED;
   if (e != cudaSuccess) return cuda_fail(e, "tlg_eval_block launch");
   g_last_family = family;
@@ -1381,6 +1423,12 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
         t->poly_staged = t->poly_bytes <= 32 * 1024 ? t->poly_bytes : t->poly_planes;
         t->off_poly = (uint32_t)align16(host_bytes);
         host_bytes = (size_t)t->off_poly + t->poly_bytes;
+        if (df && td == 3) {
+          t->polydf_points = (uint32_t)(prule.lines.size() * sizeof(tlg::PolyDfNode));
+          t->polydf_bytes = (uint32_t)align16(t->polydf_points + prule.points.size() * sizeof(tlg::PolyDfNode));
+          t->off_polydf = (uint32_t)align16(host_bytes);
+          host_bytes = (size_t)t->off_polydf + t->polydf_bytes;
+        }
       }
     }
     t->host.assign(host_bytes, 0);
@@ -1404,6 +1452,20 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
       std::memcpy(base + t->poly_planes, prule.planes.data(), prule.planes.size() * sizeof(tlg::PolyNode));
       std::memcpy(base + t->poly_lines, prule.lines.data(), prule.lines.size() * sizeof(tlg::PolyNode));
       std::memcpy(base + t->poly_points, prule.points.data(), prule.points.size() * sizeof(tlg::PolyNode));
+    }
+    if (t->polydf_bytes > 0) {
+      auto pair = [](double v) { return make_float2((float)v, (float)(v - (double)(float)v)); };
+      auto write = [&](const std::vector<tlg::PolyNode>& nodes, size_t off) {
+        auto* dst = reinterpret_cast<tlg::PolyDfNode*>(t->host.data() + t->off_polydf + off);
+        for (size_t i = 0; i < nodes.size(); ++i) {
+          const tlg::PolyNode& n = nodes[i];
+          tlg::PolyDfNode d = {pair(n.t), pair(n.t * n.s1), pair(n.t * n.t * n.t), pair(n.s2), pair(3.0 * n.t * n.t),
+                               n.first, n.count, n.plane, n.mid};
+          dst[i] = d;
+        }
+      };
+      write(prule.lines, 0);
+      write(prule.points, t->polydf_points);
     }
     if (t->sf_ok) {
       std::memcpy(t->host.data() + t->off_sf, heads.data(), heads.size() * sizeof(tlg::SfBlock));
@@ -1625,12 +1687,12 @@ tlg_status eval_dispatch(const tlg_tables* t, const tlg_block* b, const tlg_outp
   // A forced strategy that does not apply runs the loops kernel (strategy.rs:400-404); AUTO
   // falls through to the unrolled kernels, then the loops kernel over staged tables.
   const bool is_auto = strategy == TLG_STRATEGY_AUTO;
-  // f64 cells with a polynomial kernel: it is the sum factorisation of tensor rules (recorded so)
-  // and the direct kernel of the others.
-  if (t->poly_bytes > 0 && !t->df && (is_auto || strategy == TLG_STRATEGY_DIRECT || (strategy == TLG_STRATEGY_SUMFACT && t->sf_ok))) {
+  // f64 and double-float cells with a polynomial kernel: it is the sum factorisation of tensor rules
+  // (recorded so) and the direct kernel of the others.
+  if (t->poly_bytes > 0 && (is_auto || strategy == TLG_STRATEGY_DIRECT || (strategy == TLG_STRATEGY_SUMFACT && t->sf_ok))) {
     bool found = false;
-    const bool sf = t->sf_ok && strategy != TLG_STRATEGY_DIRECT;
-    tlg_status st = eval_poly(t, b, o, mask, sf ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT, s, &found);
+    const int ran = t->sf_ok && strategy != TLG_STRATEGY_DIRECT ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT;
+    tlg_status st = t->df ? eval_dfpoly(t, b, o, mask, ran, s, &found) : eval_poly(t, b, o, mask, ran, s, &found);
     if (found) return st;
   }
   if (strategy == TLG_STRATEGY_SUMFACT || (is_auto && sumfact_preferred(t))) {

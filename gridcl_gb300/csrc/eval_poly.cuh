@@ -143,9 +143,9 @@ __device__ __forceinline__ double poly_der_n(int deg, const double* A, const Pol
 }
 
 // The three stages of one item, each with its middle point's form: P_ab and Q_ab of a plane and
-// coordinate (stride between the coefficients of c and the sums of o), the line's A, D and E from
+// coordinate (strides between the coefficients of c and the sums of o), the line's A, D and E from
 // them, and X and J at a point.
-template <int CELL, int P, int STRIDE, bool AT_MID>
+template <int CELL, int P, int STRIDE, bool AT_MID, int OSTRIDE = STRIDE>
 __device__ __forceinline__ void poly_plane(const double* c, const PolyAt& z, bool want_j, double* o) {
   using S = PolySpace<CELL, P>;
 #pragma unroll
@@ -156,8 +156,8 @@ __device__ __forceinline__ void poly_plane(const double* c, const PolyAt& z, boo
 #pragma unroll
       for (int l = 0; l <= P; ++l)
         if (l <= S::cc(x, b) && (!AT_MID || l < 2)) v[l] = c[S::ci(x, b, l) * STRIDE];
-      o[S::pi(x, b) * STRIDE] = poly_val_n<P, AT_MID>(S::cc(x, b), v, z);
-      if (want_j && S::cc(x, b) > 0) o[(S::AB + S::qi(x, b)) * STRIDE] = poly_der_n<P, AT_MID>(S::cc(x, b), v, z);
+      o[S::pi(x, b) * OSTRIDE] = poly_val_n<P, AT_MID>(S::cc(x, b), v, z);
+      if (want_j && S::cc(x, b) > 0) o[(S::AB + S::qi(x, b)) * OSTRIDE] = poly_der_n<P, AT_MID>(S::cc(x, b), v, z);
     }
 }
 

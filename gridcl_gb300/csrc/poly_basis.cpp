@@ -128,6 +128,7 @@ PolyRule poly_rule(int cell, int degree, const double* points, int64_t npoints) 
         for (int e = 0; e < len; ++e) {
           PolyNode pt = poly_node(cell, degree, 0, points[l.q[at + e] * td], kLine);
           pt.first = l.q[at + e];
+          pt.plane = (int)r.lines.size();
           r.points.push_back(pt);
         }
         r.lines.push_back(ln);

@@ -19,7 +19,7 @@ struct PolyTerms {
 };
 
 // A coordinate value with what it heads: a plane (z; its lines), a line (y; its points, its plane)
-// or a point (x; `first` its index in the point set). t is the value about the direction's centre,
+// or a point (x; `first` its index in the point set, `plane` its line). t is the value about the direction's centre,
 // e_2(t) = t s1, e_2'(t) = s2; mid: t = 0 (an integer, as a comparison of doubles takes the FP64 pipe).
 struct PolyNode {
   double t, s1, s2;

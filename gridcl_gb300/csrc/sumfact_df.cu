@@ -47,10 +47,7 @@ cudaError_t launch_sumfact_df3(int n, const SfArgs& a, size_t smem, cudaStream_t
   *found = true;
   // Ten cells per warp: the persistent grid covers padded / 10 warps.
   const int64_t work = (a.padded + 9) / 10 * 32;
-  // Register caps: three CTAs per SM at Q2 (168 registers; 220 without a cap ran 8.26 ms against
-  // 7.34 ms on 128^3 Q2 hexahedra, 128 registers 7.27 ms with 276 bytes of spills).
-  if (n == 2) return launch_persistent(sumfact_df3_kernel<2, 3>, a, work, smem, s);
-  if (n == 3) return launch_persistent(sumfact_df3_kernel<3, 3>, a, work, smem, s);
+  // (Q1 and Q2 run the polynomial kernel of eval_dfpoly.cuh.)
   if (n == 4) return launch_persistent(sumfact_df3_kernel<4, 2>, a, work, smem, s);
   *found = false;
   return cudaSuccess;
