@@ -20,7 +20,7 @@ CSRC = HERE / "csrc"
 OUT_DIR = HERE / "_build"
 LIB = HERE / "libtlgeom.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["api.cu", "coop.cu", "csr.cu", "eval_df.cu", "eval_dfpoly.cu", "eval_f32.cu", "eval_f64.cu", "eval_pair.cu", "eval_poly.cu", "eval_pair_meas.cu", "measure.cu", "order.cpp", "poly_basis.cpp",
+SOURCES = ["api.cu", "coop.cu", "csr.cu", "eval_df.cu", "eval_dfpoly.cu", "eval_f32.cu", "eval_f64.cu", "eval_hexline.cu", "eval_pair.cu", "eval_poly.cu", "eval_pair_meas.cu", "measure.cu", "order.cpp", "poly_basis.cpp",
            "pullback.cu", "pullback_poly_f32.cu", "pullback_poly_f64.cu", "pullback_poly_split.cu", "refcell.cpp", "sumfact.cu", "sumfact_df.cu", "sumfact_fn.cu", "tc.cu", "umma.cu", "vjp_f64.cu", "vjp_poly.cu", "vjp_split.cu", "vjp_surface.cu"]
 
 

@@ -28,6 +28,7 @@
 #include "sumfact.cuh"
 #include "eval_df.cuh"
 #include "eval_dfpoly.cuh"
+#include "eval_hexline.cuh"
 #include "eval_poly.cuh"
 #include "poly_basis.h"
 #include "sumfact_df.cuh"
@@ -108,6 +109,9 @@ struct tlg_tables {
   uint32_t off_poly = 0, poly_bytes = 0, poly_staged = 0, poly_starts = 0, poly_tterms = 0, poly_tstarts = 0;
   uint32_t poly_planes = 0, poly_lines = 0, poly_points = 0;
   int poly_nplanes = 0, poly_nlines = 0, poly_plane_lines = 0;  // (the most lines of a plane)
+  // The section of f32 and split hexahedra Q1-Q2 in its place (eval_hexline.cuh).
+  uint32_t hexline_bytes = 0;
+  int hexline_plane = 0;  // the most points of a plane
   // Double-float tables: the rule's lines and points as PolyDfNode.
   uint32_t off_polydf = 0, polydf_bytes = 0, polydf_points = 0;
   int* err = nullptr;
@@ -535,6 +539,49 @@ tlg_status eval_poly(const tlg_tables* t, const tlg_block* b, const tlg_outputs*
   if (!*found) return TLG_ERR_UNSUPPORTED;
   if (e != cudaSuccess) return cuda_fail(e, "tlg_eval_block launch");
   g_last_family = family;
+  return ok();
+}
+
+// The FP32 line kernel of hexahedra (f32 meshes at any tile, split precision at tile 16; no facet normals);
+// `found` is false where it does not apply.
+tlg_status eval_hexline(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o, uint32_t mask,
+                        cudaStream_t stream, bool* found) {
+  *found = false;
+  const bool split = t->dtype == TLG_SPLIT32;
+  // (Rules whose table would cost resident CTAs, and in split precision planes of more points than the kernel's
+  // mask of near-degenerate ones has bits, stay with the other kernels.)
+  if (t->hexline_bytes == 0 || t->hexline_bytes > 16 * 1024 || (split && t->hexline_plane > 64) || (mask & tlg::kOutFacetNormals) || (split && o->tile != 16))
+    return TLG_ERR_UNSUPPORTED;
+  tlg::HexLineArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.nodes = b->nodes;
+  a.dofmap = b->dofmap;
+  a.tab = t->dev + t->off_poly;
+  a.dphi64 = split ? reinterpret_cast<const double*>(t->dev + t->off_dphi64) : nullptr;
+  void* outs[4] = {o->points, o->jacobian, o->detj, o->pinv};
+  for (int i = 0; i < 4; ++i) a.out[i] = static_cast<float*>(outs[i]);
+  a.err = t->err;
+  a.recomputed = o->recomputed;
+  a.first_cell = o->first_cell;
+  a.padded = (o->num_cells + o->tile - 1) / o->tile * o->tile;
+  a.range_cells = o->num_cells;
+  a.out_first_cell = o->out_first_cell;
+  a.last_cell = b->num_cells - 1;
+  for (int g = 0; g < 3; ++g) a.origin[g] = b->origin[g];
+  a.cond_limit = o->cond_limit > 0 ? (float)o->cond_limit : 256.0f;
+  a.last_node = (uint32_t)(b->num_nodes - 1);
+  a.tab_bytes = t->hexline_bytes;
+  a.off_planes = t->poly_planes;
+  a.off_lines = t->poly_lines;
+  a.off_points = t->poly_points;
+  a.mask = mask;
+  a.num_points = (int)t->q;
+  a.num_planes = t->poly_nplanes;
+  a.tile_shift = tile_shift(o->tile);
+  cudaError_t e = tlg::launch_eval_hexline(split, t->degree, a, stream, found);
+  if (!*found) return TLG_ERR_UNSUPPORTED;
+  if (e != cudaSuccess) return cuda_fail(e, "tlg_eval_block launch");
+  g_last_family = TLG_STRATEGY_DIRECT;
   return ok();
 }
 
@@ -1431,7 +1478,37 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
         }
       }
     }
+    // Hexahedra Q1-Q2 in f32 and split precision: the lattice, then the rule's planes, lines and points in f32.
+    if (dtype != TLG_F64 && cell == tlg::kHexahedron && degree <= 2 && npoints > 0) {
+      std::vector<double> s1, lt;
+      if (sf_permutation(cell, degree, family, s1, lt, pstarts)) {
+        prule = tlg::poly_rule(cell, degree, points, npoints);
+        t->poly_nplanes = (int)prule.planes.size();
+        std::vector<int> of_plane(prule.planes.size(), 0);
+        for (const tlg::PolyNode& l : prule.lines) t->hexline_plane = std::max(t->hexline_plane, of_plane[l.plane] += l.count);
+        t->poly_planes = (uint32_t)align16(pstarts.size() * 4);
+        t->poly_lines = (uint32_t)(t->poly_planes + prule.planes.size() * sizeof(tlg::PolyNodeF));
+        t->poly_points = (uint32_t)(t->poly_lines + prule.lines.size() * sizeof(tlg::PolyNodeF));
+        t->hexline_bytes = (uint32_t)(t->poly_points + prule.points.size() * sizeof(tlg::PolyNodeF));
+        t->off_poly = (uint32_t)align16(host_bytes);
+        host_bytes = (size_t)t->off_poly + t->hexline_bytes;
+      }
+    }
     t->host.assign(host_bytes, 0);
+    if (t->hexline_bytes > 0) {
+      unsigned char* base = t->host.data() + t->off_poly;
+      std::memcpy(base, pstarts.data(), pstarts.size() * 4);
+      auto write = [&](const std::vector<tlg::PolyNode>& nodes, size_t off) {
+        auto* dst = reinterpret_cast<tlg::PolyNodeF*>(base + off);
+        for (size_t i = 0; i < nodes.size(); ++i) {
+          const tlg::PolyNode& n = nodes[i];
+          dst[i] = {(float)n.t, (float)n.s1, (float)n.s2, n.mid, n.first, n.count, n.plane, 0};
+        }
+      };
+      write(prule.planes, t->poly_planes);
+      write(prule.lines, t->poly_lines);
+      write(prule.points, t->poly_points);
+    }
     if (t->poly_bytes > 0) {
       unsigned char* base = t->host.data() + t->off_poly;
       if (!pterms.empty()) std::memcpy(base, pterms.data(), pterms.size() * sizeof(tlg::PolyTerm));
@@ -1693,6 +1770,11 @@ tlg_status eval_dispatch(const tlg_tables* t, const tlg_block* b, const tlg_outp
     bool found = false;
     const int ran = t->sf_ok && strategy != TLG_STRATEGY_DIRECT ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT;
     tlg_status st = t->df ? eval_dfpoly(t, b, o, mask, ran, s, &found) : eval_poly(t, b, o, mask, ran, s, &found);
+    if (found) return st;
+  }
+  if (t->hexline_bytes > 0 && (is_auto || strategy == TLG_STRATEGY_DIRECT)) {
+    bool found = false;
+    tlg_status st = eval_hexline(t, b, o, mask, s, &found);
     if (found) return st;
   }
   if (strategy == TLG_STRATEGY_SUMFACT || (is_auto && sumfact_preferred(t))) {

@@ -1,0 +1,22 @@
+// Instantiations of the FP32 line kernel of hexahedra.
+#include "eval_hexline.cuh"
+
+namespace tlg {
+
+template <bool SPLIT, int P>
+static cudaError_t launch_degree(const HexLineArgs& a, cudaStream_t s) {
+  const size_t smem = a.tab_bytes + (size_t)(P + 1) * (P + 1) * (P + 1) * 3 * kEvalThreads * 4;
+  if (a.tile_shift == 4) return launch_persistent(eval_hexline_kernel<SPLIT, P, 4>, a, a.padded, smem, s);
+  if constexpr (!SPLIT) return launch_persistent(eval_hexline_kernel<SPLIT, P, -1>, a, a.padded, smem, s);
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_eval_hexline(bool split, int degree, const HexLineArgs& a, cudaStream_t s, bool* found) {
+  *found = true;
+  if (degree == 1) return split ? launch_degree<true, 1>(a, s) : launch_degree<false, 1>(a, s);
+  if (degree == 2) return split ? launch_degree<true, 2>(a, s) : launch_degree<false, 2>(a, s);
+  *found = false;
+  return cudaSuccess;
+}
+
+}  // namespace tlg
