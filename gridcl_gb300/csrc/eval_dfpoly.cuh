@@ -88,9 +88,10 @@ using Dp = DF<float2>;
 // double the kernel's code for values that are rarely special.
 static __device__ __noinline__ void df_pairs_slow(float4* t, int n) {
   for (int c = 0; c < n; ++c) {
-    // (An infinite or NaN head has a NaN tail: its f64 is the head's.)
-    const double x = isfinite(t[c].x) ? df_to_f64(t[c].x, t[c].z) : (double)t[c].x;
-    const double y = isfinite(t[c].y) ? df_to_f64(t[c].y, t[c].w) : (double)t[c].y;
+    // (An infinite or NaN head has a NaN tail: left out.)
+    const float lx = (__float_as_uint(t[c].x) << 1) >= 0xFF000000u ? 0.0f : t[c].z;
+    const float ly = (__float_as_uint(t[c].y) << 1) >= 0xFF000000u ? 0.0f : t[c].w;
+    const double x = df_to_f64(t[c].x, lx), y = df_to_f64(t[c].y, ly);
     t[c] = make_float4(__int_as_float(__double2hiint(x)), __int_as_float(__double2loint(x)),
                        __int_as_float(__double2hiint(y)), __int_as_float(__double2loint(y)));
   }
