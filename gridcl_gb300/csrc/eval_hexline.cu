@@ -6,7 +6,11 @@ namespace tlg {
 template <bool SPLIT, int P>
 static cudaError_t launch_degree(const HexLineArgs& a, cudaStream_t s) {
   const size_t smem = a.tab_bytes + (size_t)(P + 1) * (P + 1) * (P + 1) * 3 * kEvalThreads * 4;
-  if (a.tile_shift == 4) return launch_persistent(eval_hexline_kernel<SPLIT, P, 4>, a, a.padded, smem, s);
+  // One step per CTA for f32 Q1 (8 points, 1,500,000 cells: 0.200 ms persistent, 0.175 so); f32 Q2 at 27 points
+  // is even (500,000 cells 0.239 / 0.232, 100,000 0.061 / 0.065), split precision slower (Q2 0.338 / 0.352, Q1
+  // 0.216 / 0.261).
+  if (a.tile_shift == 4)
+    return launch_persistent(eval_hexline_kernel<SPLIT, P, 4>, a, a.padded, smem, s, P == 1 && !SPLIT);
   if constexpr (!SPLIT) return launch_persistent(eval_hexline_kernel<SPLIT, P, -1>, a, a.padded, smem, s);
   return cudaErrorInvalidValue;
 }

@@ -49,15 +49,21 @@ inline int persistent_grid(Kernel kern, size_t smem, int64_t work_items, int thr
   return (int)(need < cap ? (need > 0 ? need : 1) : cap);
 }
 
+// The grid-stride kernels run persistent CTAs, or with `one_step` a CTA per kEvalThreads cells (the
+// autotuner's grid either way). One step per CTA costs a table copy each, but CTAs start as others end:
+// the warps of an SM spread over the gather, the sums and the stores, where persistent CTAs pass through
+// them together. It is the faster where a cell's start (index and coordinate loads, split precision's FP64
+// subtractions) is small beside its stores; the callers' rules give the measurements.
 template <typename Kernel, typename Args>
 inline cudaError_t launch_persistent(Kernel kern, const Args& a, int64_t work, size_t smem,
-                                     cudaStream_t s) {
+                                     cudaStream_t s, bool one_step = false) {
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  const int grid = persistent_grid(kern, smem, work, kEvalThreads);
-  kern<<<grid, kEvalThreads, smem, s>>>(a);
+  int64_t grid = (work + kEvalThreads - 1) / kEvalThreads;
+  if (!one_step || g_grid_override > 0 || grid < 1) grid = persistent_grid(kern, smem, work, kEvalThreads);
+  kern<<<(unsigned)grid, kEvalThreads, smem, s>>>(a);
   return cudaGetLastError();
 }
 
