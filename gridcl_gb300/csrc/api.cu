@@ -25,6 +25,7 @@
 #include "coop.cuh"
 #include "tc.cuh"
 #include "umma.cuh"
+#include "umma_rows.cuh"
 #include "sumfact.cuh"
 #include "eval_df.cuh"
 #include "eval_dfpoly.cuh"
@@ -723,10 +724,14 @@ tlg_status eval_umma(const tlg_tables* t, const tlg_block* b, const tlg_outputs*
   if (t->umma_kpad == 0 || o->tile != 16 || (t->dtype != TLG_F32 && t->dtype != TLG_SPLIT32) ||
       (mask & tlg::kOutNormals))
     return TLG_ERR_UNSUPPORTED;
-  // At least 80 KiB, so that at most two CTAs (2 x 256 tensor-memory columns) share an SM.
-  const size_t smem = std::max<size_t>(tlg::umma_smem_bytes(t->umma_kpad), (size_t)80 * 1024);
-  if (smem > (size_t)227 * 1024) return TLG_ERR_UNSUPPORTED;
   const bool split = t->dtype == TLG_SPLIT32;
+  // One accumulator row per cell where 128 cells' heads and tails fit shared memory.
+  const size_t rows_smem = tlg::umma_rows_smem_bytes(t->umma_kpad, split);
+  const bool rows = t->k >= tlg::kRowsMinNodes && rows_smem <= (size_t)227 * 1024;
+  // The other kernel: at least 80 KiB, so that at most two CTAs (2 x 256 tensor-memory columns) share an SM.
+  const size_t smem = rows ? std::max(rows_smem, tlg::kRowsMinSmem)
+                           : std::max<size_t>(tlg::umma_smem_bytes(t->umma_kpad), (size_t)80 * 1024);
+  if (smem > (size_t)227 * 1024) return TLG_ERR_UNSUPPORTED;
   tlg::UmmaArgs a;
   std::memset(&a, 0, sizeof(a));
   a.nodes = b->nodes;
@@ -753,7 +758,7 @@ tlg_status eval_umma(const tlg_tables* t, const tlg_block* b, const tlg_outputs*
   a.num_points = (int)t->q;
   a.chunks = t->umma_chunks;
   *found = true;
-  cudaError_t e = tlg::launch_umma(split, a, smem, stream);
+  cudaError_t e = rows ? tlg::launch_umma_rows(split, a, smem, stream) : tlg::launch_umma(split, a, smem, stream);
   if (e != cudaSuccess) return cuda_fail(e, "tlg_eval_block launch");
   g_last_family = TLG_STRATEGY_TENSOR;
   return ok();

@@ -1,5 +1,6 @@
 // Blackwell tensor-core evaluation (tcgen05) for volume cells of many nodes: the node-by-basis
-// contraction X^T Phi as a UMMA with FP32 accumulators in tensor memory.
+// contraction X^T Phi as a UMMA with FP32 accumulators in tensor memory. The policy runs it for cells of
+// 65 to 88 nodes (64 in split precision); those of 28 to 64 nodes run the kernel of umma_rows.cuh.
 //
 // Per tile of 64 cells, for each coordinate g the A operand (M = 128 rows, K = nodes) holds the
 // TF32 heads of the cells' coordinates relative to their first node in rows 0-63 and the TF32
