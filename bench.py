@@ -49,10 +49,10 @@ METRIC = "Jacobian qpoints/s (fwd, fwd+adjoint) vs plain FP64 GPU path at stated
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of the evaluation
 # kernel on the 64^3 workload, measured on a GB300 by one-pass ncu captures of
 # `bench.py --no-extras --no-cpu-baseline --steps 3 --warmup 3 [--mode f64]` (-s 3 -c 1):
-# split eval_pair_kernel<1,3,3,10> 191.07 MB + 3.26 GB; f64 eval_direct_kernel<double,3,3,10,16>
-# 166.22 MB + 6.58 GB; double-float eval_df_kernel<3,3,10> 171.69 MB + 6.581 GB. Reported as
+# split eval_pair_kernel<1,3,3,10> 119.27 MB + 3.258 GB; f64 eval_poly_kernel<4,2,3>
+# 160.99 MB + 6.579 GB; double-float eval_dfpoly_kernel<4,2> 154.02 MB + 6.579 GB. Reported as
 # roofline.traffic, scaled by quadrature points for other n.
-NCU_TRAFFIC_64 = {"split": 191.07e6 + 3.26e9, "f64": 166.22e6 + 6.58e9, "df64": 171.69e6 + 6.581e9}
+NCU_TRAFFIC_64 = {"split": 119.27e6 + 3.258e9, "f64": 160.99e6 + 6.579e9, "df64": 154.02e6 + 6.579e9}
 QPOINTS_64 = 64 ** 3 * 6 * 24
 
 
@@ -839,9 +839,9 @@ def extra_p1_box():
 # What binds each mode's kernel, from its ncu capture (the profiles of the P2 tetrahedra): the
 # double-float and FP64 kernels are bound by an arithmetic pipe, not by HBM.
 BINDING = {
-    "df64": "FP32 pipes: FMA 54.8 %, ALU 45.5 %, issue 59.9 % of active cycles (ncu, 32^3 x 6 case, monomial form)",
-    "f64": "FP64 pipe: 93.7 % of active cycles (ncu)",
-    "split": "HBM: stores of the f32 fields (ncu traffic 1.004 x the algorithmic bytes)",
+    "df64": "issue 47 % over three pipes: FP64 39 %, ALU 38 %, FMA 32 % of active cycles (ncu, 32^3 x 6 case)",
+    "f64": "FP64 pipe: 91.0 % of active cycles (ncu)",
+    "split": "HBM: stores of the f32 fields (ncu traffic 0.98 x the algorithmic bytes)",
     "f32": "HBM: stores of the f32 fields",
 }
 # Algorithmic FP64 operations per point of the curved P2 tetrahedra (x: 3 x 10 FMAs, J: 9 x 10

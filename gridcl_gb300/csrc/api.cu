@@ -301,8 +301,8 @@ int principal_family(uint32_t mask) {
 // Q3 - / 395 / 45.4 (the FP64 pipe bounds, and sum factorisation does a third of the multiply-adds;
 // Q1-Q2 and prisms P1-P2 run the polynomial kernel under either name); split Q1 0.33 / 1.21 / 0.35, Q2 1.37 / 21.9 / 1.53,
 // Q3 - / 11.5 / 0.62; f32 Q2 1.15 / 17.6 / 1.39, Q3 - / 16.7 / 0.55. So: sum factorisation
-// always in f64, and in f32 and split precision above the degrees with paired kernels
-// (quadrilaterals and hexahedra Q1-Q2).
+// always in f64 (beyond the polynomial kernel), and in f32 and split precision above the degrees with
+// paired kernels (quadrilaterals and hexahedra Q1-Q2; hexahedra Q1-Q2 run the line kernel).
 bool sumfact_preferred(const tlg_tables* t) { return t->sf_ok && (t->dtype == TLG_F64 || t->sf_n >= 4); }
 
 // The policy of TLG_STRATEGY_AUTO beyond the compiled unrolled kernels (more than 27 nodes per
@@ -316,8 +316,8 @@ bool tc_preferred(const tlg_tables*) { return false; }
 
 // The tcgen05 kernel replaces the cooperative kernel where it applies (f32 and split tables of
 // volume cells in 3D, 27 < K <= 88). GB300, curved tetrahedra 6 x 16^3 at Gauss rules of degree
-// 2p, ms (tcgen05 / cooperative): f32 P4 0.180 / 0.197, P5 0.313 / 0.691, P6 0.629 / 1.436;
-// split P4 0.201 / 0.215, P5 0.465 / 0.765, P6 0.897 / 2.750.
+// 2p, ms (tcgen05 / cooperative): f32 P4 0.064 / 0.197, P5 0.141 / 0.676, P6 0.534 / 1.425;
+// split P4 0.119 / 0.216, P5 0.291 / 0.761, P6 0.776 / 2.746.
 bool umma_preferred(const tlg_tables* t) { return t->umma_kpad > 0 && t->k > 27; }
 
 // The sum-factorised kernel; `found` is false when it does not apply (no tensor structure, facet

@@ -14,8 +14,10 @@
 // Arithmetic follows tetraloma-geometry/src/layout.rs:133-369: J(g, d) is the sum over the
 // nodes in ascending k starting with the k = 0 product; det J and K by the same cofactor
 // formulas; normals as s (J0 x J1) / |J0 x J1|. Every operation is an explicitly rounded
-// intrinsic (no compiler contraction), written once for scalars and for f32 pairs, so the
-// kernels below give the same bits for the same point whichever of them runs.
+// intrinsic (no compiler contraction), written once for scalars and for f32 pairs, so the sums
+// (x, J, and det J and K of volume cells) have the same bits for the same point whichever of the
+// kernels below runs. Surfaces differ in the last bits: the paired kernel forms their area
+// element, normal and K from one reciprocal square root (SurfacePair).
 //
 // Kernels:
 //  - eval_pair_kernel<SPLIT, TD, GD, K>: f32 arithmetic on two quadrature points at once with
@@ -23,8 +25,10 @@
 //    SPLIT = true: an f64 mesh, each cell shifted by its node 0 in f64 before rounding to f32,
 //    f32 fields, and an FP64 recompute of J, det J and K at points whose condition estimate
 //    exceeds a limit (counted in a device counter).
-//  - eval_direct_kernel<F, TD, GD, K, TILE>: scalar, everything unrolled (the f64 path).
+//  - eval_direct_kernel<F, TD, GD, K, TILE>: scalar, everything unrolled (f64 intervals, pyramids P1-P3, P4
+//    triangles; the other f64 elements run the polynomial kernel of eval_poly.cuh).
 //  - eval_loops_kernel<F, TD, GD>: K and the tile at run time (every other element and tile).
+// Hexahedra on f32 meshes and in split precision run the line kernel of eval_hexline.cuh.
 #pragma once
 
 #include <cstdint>

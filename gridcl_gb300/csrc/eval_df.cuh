@@ -11,6 +11,9 @@
 // X adds x_0 + origin (a double-float per cell), and det J, K, normals and facet normals follow
 // in double-float by the formulas of the other kernels (Factors<DF<float2>, TD, GD>); every value
 // is assembled into its f64 (df_to_f64) and stored into its QuadField chunk.
+//
+// What reaches it: surfaces, planar cells and pyramids; of tetrahedra, hexahedra and prisms the
+// calls that ask for facet normals (the others run the polynomial kernel of eval_dfpoly.cuh).
 #pragma once
 
 #include <cstdint>

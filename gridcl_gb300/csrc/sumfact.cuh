@@ -12,6 +12,11 @@
 // with B_d[a][i] = l_i(u_d[a]) and D_d[a][i] = l_i'(u_d[a]): N^3 M (2) + N^2 M^2 (3) + N M^3 (4)
 // multiply-adds per coordinate instead of N^3 M^3 (4). Quadrilaterals contract two directions.
 //
+// What reaches it: quadrilaterals and prisms on f32 meshes and in split precision, Q3 hexahedra, P3
+// prisms and the larger quadrilaterals in every type, and hexahedra Q1-Q2 in f32 where the line kernel
+// (eval_hexline.cuh) does not apply. The smaller f64 cells contract their polynomials instead
+// (eval_poly.cuh).
+//
 // One cell per thread, as the other evaluation kernels (consecutive threads write consecutive
 // tile lanes). The cell's coordinates in lexicographic node order (the table's permutation maps
 // a lexicographic index to the Lagrange node) go to the thread's slots in shared memory,

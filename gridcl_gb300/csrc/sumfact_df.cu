@@ -1,6 +1,6 @@
 // Instantiations of the double-float sum-factorised kernels (sumfact_df.cuh): hexahedra Q1-Q3,
 // quadrilaterals Q1-Q5 (planar and embedded in 3D), prisms P1-P3, with and without facet normals,
-// and the three-lanes-per-cell hexahedra.
+// and the three-lanes-per-cell Q3 hexahedra.
 #include "eval_launch.cuh"
 #include "sumfact_df.cuh"
 

@@ -10,9 +10,11 @@
 // double-floats in registers, the point stage on point pairs (the paired FP32 instructions), and
 // each pair's det J, K, normals and facet normals follow in double-float, assembled into f64 and
 // stored.
-//  - sumfact_df_kernel: one cell per thread (quadrilaterals, Q1 hexahedra, facet normals);
-//  - sumfact_df3_kernel: hexahedra with three lanes per cell, lane g computing coordinate g;
-//  - sumfact_prism_df_kernel: prisms, one cell per thread, the z points two at a time.
+//  - sumfact_df_kernel: one cell per thread (quadrilaterals, facet normals);
+//  - sumfact_df3_kernel: Q3 hexahedra with three lanes per cell, lane g computing coordinate g;
+//  - sumfact_prism_df_kernel: prisms, one cell per thread, the z points two at a time (rules with
+//    one line of points per plane, P3, facet normals).
+// Hexahedra Q1-Q2 and the other prisms run the polynomial kernel of eval_dfpoly.cuh.
 #pragma once
 
 #include <cstdint>
