@@ -316,7 +316,7 @@ bool tc_preferred(const tlg_tables*) { return false; }
 
 // The tcgen05 kernel replaces the cooperative kernel where it applies (f32 and split tables of
 // volume cells in 3D, 27 < K <= 88). GB300, curved tetrahedra 6 x 16^3 at Gauss rules of degree
-// 2p, ms (tcgen05 / cooperative): f32 P4 0.064 / 0.197, P5 0.141 / 0.676, P6 0.534 / 1.425;
+// 2p, ms (tcgen05 / cooperative): f32 P4 0.069 / 0.196, P5 0.133 / 0.676, P6 0.534 / 1.425;
 // split P4 0.119 / 0.216, P5 0.291 / 0.761, P6 0.776 / 2.746.
 bool umma_preferred(const tlg_tables* t) { return t->umma_kpad > 0 && t->k > 27; }
 

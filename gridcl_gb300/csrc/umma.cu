@@ -38,7 +38,7 @@ cudaError_t launch_umma(bool split, const UmmaArgs& args, size_t smem, cudaStrea
 
 // The kernel cuts the (tile, chunk) pairs, in tile order, into equal runs, one per CTA (one CTA fits an
 // SM). A run costs its chunks and, for every tile that it touches, a start (the gather and the first MMAs)
-// of about eight chunks: P5 tetrahedra on an f32 mesh take 2.55 us a chunk and 20 us a start. So the grid
+// of six to eight chunks: P5 tetrahedra on an f32 mesh take 2.5 us a chunk and 15 us a start. So the grid
 // is every SM, unless whole tiles or whole parts of a tile per CTA on fewer SMs cost less: of T tiles of n
 // chunks on C SMs, ceil(T / C) (n + 8) where T > C, ceil(n / floor(C / T)) + 8 else, against
 // r + 8 (floor((r - 1) / n) + 2), r = ceil(T n / C). GB300, us, equal runs / whole ones: P4 f32, 24 tiles
@@ -48,7 +48,7 @@ cudaError_t launch_umma_rows(bool split, const UmmaArgs& a, size_t smem, cudaStr
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   constexpr int64_t kStart = 8;
-  const int threads = rows_threads(split);
+  const int threads = kRowsThreads;
   const int64_t tiles = (a.padded + kRowsCells - 1) / kRowsCells, n = a.chunks;
   const int64_t ctas = persistent_grid(kern, smem, tiles * n * threads, threads);
   int64_t grid = ctas;

@@ -11,7 +11,7 @@
 // row's head column and tail column.
 //
 // Bound: every partial product of a cell lands in the lane that stores the cell, so the epilogue (one
-// thread per cell, sixteen warps of two points a chunk) needs no exchange and no CTA-wide barrier. Warps
+// thread per cell, eight warps of four points a chunk) needs no exchange and no CTA-wide barrier. Warps
 // wait for a chunk's accumulators (mbarrier), load them, release the buffer (mbarrier, one arrival per
 // warp) and finish their points; a seventeenth warp issues the table copies and the MMAs, a chunk
 // ahead of the epilogue. N = 64 because the MMAs of this shape are bound by reading A (66 cycles for
@@ -21,15 +21,15 @@
 // beside the heads, and of fewer (forced strategies; two of its CTAs fit an SM).
 //
 // GB300, ms, that kernel / this one (all four factors): P5 tetrahedra, 216 points, 24,576 cells, f32 0.255
-// / 0.149 (a floor of 0.071 by bytes), split 0.287 / 0.178; 19,456 cells (a tile per SM) 0.174 / 0.090, split
-// 0.195 / 0.099; P4, 125 points, 90,000 cells, f32 0.438 / 0.224, split 0.505 / 0.285; 3,000 cells 0.023 /
-// 0.016. Error against 64 bits on the first: 1.4e-6 / 9.6e-7 (fewer products meet in one accumulator). What
-// is left there: a chunk takes 2.55 us, 2.1 of them the 42 MMAs (with one output alone), a tile's start 20 us.
-// On the way, same case: one thread issuing behind a thread-index test, a coordinate after the other,
-// work items in groups as in the other kernel 0.178; a converged warp electing the issuing lane 0.149;
-// equal runs even at first (a 64-bit remainder per copy), 0.145-0.149 (launch_umma_rows). Split precision
-// with sixteen warps of 96 registers spilled: 0.312; eight warps of 168 0.216; two node quads a round in
-// the gather 0.191 (f32 has no registers for it: 0.155 with, 0.149 without).
+// / 0.133 (a floor of 0.071 by bytes), split 0.287 / 0.178; 19,456 cells (a tile per SM) 0.174 / 0.083, split
+// 0.195 / 0.099; P4, 125 points, 90,000 cells, f32 0.438 / 0.219, split 0.505 / 0.285; 3,000 cells 0.023 /
+// 0.017. Error against 64 bits on the first: 1.4e-6 / 9.6e-7 (fewer products meet in one accumulator). What
+// is left there: a chunk takes 2.5 us, 2.0 of them the 42 MMAs (with one output alone), a tile's start 15 us.
+// On the way, same case: one thread issuing behind a thread-index test, a coordinate after the other, work
+// items in groups as in the other kernel 0.178; a converged warp electing the issuing lane, coordinates
+// interleaved, equal runs 0.149, all with sixteen epilogue warps of 96 registers and one node quad a round
+// of the gather (two spilled: 0.155); eight warps of 168 registers with two quads 0.139, four 0.133. Split:
+// sixteen warps (spills) 0.312, eight 0.216, two quads 0.191, equal runs 0.178; three quads spill: 0.197.
 //
 // Tensor memory: 2 buffers x 3 coordinates x 64 columns, 512 allocated; the launch asks for at least 152
 // KB of shared memory, so that no other CTA of a tensor-memory kernel shares the SM and the allocation
@@ -44,8 +44,8 @@ namespace tlg {
 
 constexpr int kRowsCells = 128;                      // cells per tile
 // Epilogue warps (a quarter of them per lane quarter, two points at a time), and the issuing warp.
-__host__ __device__ constexpr int rows_epi_warps(bool split) { return split ? 8 : 16; }
-__host__ __device__ constexpr int rows_threads(bool split) { return rows_epi_warps(split) * 32 + 32; }
+constexpr int kRowsEpiWarps = 8;
+constexpr int kRowsThreads = kRowsEpiWarps * 32 + 32;
 constexpr int kRowsN = 2 * kUmmaN;                   // columns per coordinate: heads, tails
 constexpr int kRowsTmemCols = 512;
 constexpr int kRowsMinNodes = 28;                    // fewer nodes: the kernel of umma.cuh
@@ -125,9 +125,9 @@ static __device__ __noinline__ void umma_recompute_point(const UmmaArgs& a, int6
 cudaError_t launch_umma_rows(bool split, const UmmaArgs& a, size_t smem, cudaStream_t s);
 
 template <bool SPLIT>
-__global__ void __launch_bounds__(rows_threads(SPLIT), 1) umma_rows_kernel(const __grid_constant__ UmmaArgs a) {
+__global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const __grid_constant__ UmmaArgs a) {
   constexpr int TD = 3, GD = 3, LJ = 9;
-  constexpr int kEpi = rows_epi_warps(SPLIT), kPart = kEpi / 4;  // kPart warps share a lane quarter
+  constexpr int kEpi = kRowsEpiWarps, kPart = kEpi / 4;  // kPart warps share a lane quarter
   using A = Ar<float>;
   using M = Factors<float, TD, GD>;
   using NT = typename std::conditional<SPLIT, double, float>::type;
@@ -262,10 +262,10 @@ __global__ void __launch_bounds__(rows_threads(SPLIT), 1) umma_rows_kernel(const
       const uint32_t n0 = min(__ldg(row), a.last_node);
 #pragma unroll
       for (int g = 0; g < GD; ++g) x0[g] = __ldg(nodes + (int64_t)n0 * GD + g);
-      // The next quads' indices are loaded ahead, so that a round waits for its coordinates only; two
-      // quads a round in split precision (its 8 warps have the registers). (Beyond the cell's nodes: its
-      // first node, its coordinates taken as zero.)
-      constexpr int kQuads = SPLIT ? 2 : 1;
+      // The next quads' indices are loaded ahead, so that a round waits for its coordinates only; as many
+      // quads a round as the registers hold. (Beyond the cell's nodes: its first node, its coordinates
+      // taken as zero.)
+      constexpr int kQuads = SPLIT ? 2 : 4;
       auto load_indices = [&](int kq, uint32_t (*n)[4]) {
 #pragma unroll
         for (int h = 0; h < kQuads; ++h)
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(rows_threads(SPLIT), 1) umma_rows_kernel(const
       if (nfix > 0) {  // the same for the CTA
         __syncthreads();
         if (tid == 0) *fix_n = 0;  // the next item's gather ends with a barrier
-        for (int e = tid; e < nfix; e += rows_threads(SPLIT))  // the issuing warp too
+        for (int e = tid; e < nfix; e += kRowsThreads)  // the issuing warp too
           umma_recompute_point(a, tile * kRowsCells + (fix[e] >> 16), (int)(fix[e] & 0xFFFFu));
       }
     }
