@@ -384,8 +384,7 @@ inline cudaError_t launch_dfpoly_cell(PolyDfArgs a, int lines, cudaStream_t s) {
   while (a.chunk > 8 && bytes(a.batch, a.chunk) > 64 * 1024) a.chunk = (a.chunk + 1) / 2;
   a.alias = a.batch >= planes ? 1 : 0;
   const size_t smem = bytes(a.batch, a.chunk);
-  cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return e;
   const int64_t ctas = (a.padded + 15) / 16;
   // CTAs of 64 threads (few threads at a barrier, many CTAs), or of 96 where a batch's (point, pair)

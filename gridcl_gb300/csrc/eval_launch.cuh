@@ -49,6 +49,19 @@ inline int persistent_grid(Kernel kern, size_t smem, int64_t work_items, int thr
   return (int)(need < cap ? (need > 0 ? need : 1) : cap);
 }
 
+// Lets launches of `kern` take `smem` bytes of dynamic shared memory. The default limit of 48 KiB holds for
+// the dynamic and the static bytes together, and the kernels launched this way declare up to 400 static
+// ones (barriers, cell offsets): a dynamic size just below 48 KiB needs the attribute too. The limit is
+// set to the same value whatever the size, so that threads launching one kernel with different tables
+// do not lower it under each other.
+constexpr size_t kStaticSmemMost = 1024, kDynamicSmemMost = (size_t)227 * 1024 - kStaticSmemMost;
+template <typename Kernel>
+inline cudaError_t allow_smem(Kernel kern, size_t smem) {
+  if (smem + kStaticSmemMost <= (size_t)48 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(smem > kDynamicSmemMost ? smem : kDynamicSmemMost));
+}
+
 // The grid-stride kernels run persistent CTAs, or with `one_step` a CTA per kEvalThreads cells (the
 // autotuner's grid either way). One step per CTA costs a table copy each, but CTAs start as others end:
 // the warps of an SM spread over the gather, the sums and the stores, where persistent CTAs pass through
@@ -57,10 +70,8 @@ inline int persistent_grid(Kernel kern, size_t smem, int64_t work_items, int thr
 template <typename Kernel, typename Args>
 inline cudaError_t launch_persistent(Kernel kern, const Args& a, int64_t work, size_t smem,
                                      cudaStream_t s, bool one_step = false) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  cudaError_t e = allow_smem(kern, smem);
+  if (e != cudaSuccess) return e;
   int64_t grid = (work + kEvalThreads - 1) / kEvalThreads;
   if (!one_step || g_grid_override > 0 || grid < 1) grid = persistent_grid(kern, smem, work, kEvalThreads);
   kern<<<(unsigned)grid, kEvalThreads, smem, s>>>(a);

@@ -469,8 +469,7 @@ inline cudaError_t launch_poly_width(PolyEvalArgs a, int lines, cudaStream_t s) 
   const size_t value_bytes = (size_t)GD * W * 8;
   const size_t smem = a.cells.tab_bytes + (size_t)(tensor ? 1 : 2) * S::K * value_bytes +
                       (S::TD == 3 ? (size_t)a.batch * S::PLANE * value_bytes : 0);
-  cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return e;
   const int64_t ctas = (a.padded + W - 1) / W;
   const int in_batch = (int)((int64_t)lines * std::min(a.batch, a.num_planes) / std::max(a.num_planes, 1));

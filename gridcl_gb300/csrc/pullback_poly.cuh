@@ -388,8 +388,7 @@ inline int poly_threads(int nq) {
 
 template <typename Kernel>
 inline cudaError_t launch_poly(Kernel kern, const PolyArgs& a, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return e;
   const int64_t ctas = (a.p.padded + kPolyCells - 1) / kPolyCells;
   kern<<<(unsigned)ctas, poly_threads(a.p.num_points), smem, s>>>(a);

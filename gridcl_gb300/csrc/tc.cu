@@ -11,10 +11,8 @@ cudaError_t launch_tc(bool split, int td, int gd, const TcArgs& a, size_t smem, 
 #define TLG_TC(SPLIT, TD, GD) \
   if (split == SPLIT && td == TD && gd == GD) { \
     auto kern = tc_eval_kernel<SPLIT, TD, GD>; \
-    if (smem > 48 * 1024) { \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      if (e != cudaSuccess) return e; \
-    } \
+    cudaError_t e = allow_smem(kern, smem); \
+    if (e != cudaSuccess) return e; \
     const int grid = persistent_grid(kern, smem, warps * 32, kTcWarps * 32); \
     kern<<<grid, kTcWarps * 32, smem, s>>>(a); \
     return cudaGetLastError(); \

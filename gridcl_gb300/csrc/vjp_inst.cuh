@@ -10,10 +10,8 @@ cudaError_t TLG_VJP_LAUNCH(int d, int k, const VjpArgs& a, size_t smem, cudaStre
 #define TLG_VJP(D, K) \
   if (d == D && k == K) { \
     auto kern = vjp_kernel<TLG_VJP_SPLIT, D, K>; \
-    if (smem > 48 * 1024) { \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      if (e != cudaSuccess) return e; \
-    } \
+    cudaError_t e = allow_smem(kern, smem); \
+    if (e != cudaSuccess) return e; \
     const int grid = persistent_grid(kern, smem, a.padded * kVjpGroup, kEvalThreads); \
     kern<<<grid, kEvalThreads, smem, s>>>(a); \
     return cudaGetLastError(); \

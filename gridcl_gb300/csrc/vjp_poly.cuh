@@ -417,7 +417,7 @@ inline cudaError_t launch_vjp_poly_width(VjpPolyArgs a, int lines, cudaStream_t 
   while (a.chunk > 2 && bytes(a.batch, a.chunk) > budget) --a.chunk;
   a.alias = S::TD == 3 && a.chunk * W <= 192 && a.chunk >= in_batch(a.batch) ? 1 : 0;
   const size_t smem = bytes(a.batch, a.chunk);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return e;
   const int64_t ctas = (a.padded + W - 1) / W;
   kern<<<(unsigned)ctas, poly_line_threads(a.chunk * W, 192), smem, s>>>(a);
