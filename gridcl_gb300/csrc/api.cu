@@ -107,14 +107,16 @@ struct tlg_tables {
   // Polynomial section (f64 tables of cells of degree 1-3, eval_poly.cuh; 0 bytes elsewhere): the
   // expansion's terms and row starts (tensor cells: the lattice's nodes in the starts), the same by
   // column, the rule's planes, lines and points; the first poly_staged bytes go to shared memory.
-  uint32_t off_poly = 0, poly_bytes = 0, poly_staged = 0, poly_starts = 0, poly_tterms = 0, poly_tstarts = 0;
+  uint64_t off_poly = 0;
+  uint32_t poly_bytes = 0, poly_staged = 0, poly_starts = 0, poly_tterms = 0, poly_tstarts = 0;
   uint32_t poly_planes = 0, poly_lines = 0, poly_points = 0;
   int poly_nplanes = 0, poly_nlines = 0, poly_plane_lines = 0;  // (the most lines of a plane)
   // The section of f32 and split hexahedra Q1-Q2 in its place (eval_hexline.cuh).
   uint32_t hexline_bytes = 0;
   int hexline_plane = 0;  // the most points of a plane
   // Double-float tables: the rule's lines and points as PolyDfNode.
-  uint32_t off_polydf = 0, polydf_bytes = 0, polydf_points = 0;
+  uint64_t off_polydf = 0;
+  uint32_t polydf_bytes = 0, polydf_points = 0;
   int* err = nullptr;
   std::vector<unsigned char> host;  // host copy of the device bytes
 };
@@ -549,9 +551,9 @@ tlg_status eval_hexline(const tlg_tables* t, const tlg_block* b, const tlg_outpu
                         cudaStream_t stream, bool* found) {
   *found = false;
   const bool split = t->dtype == TLG_SPLIT32;
-  // (Rules whose table would cost resident CTAs, and in split precision planes of more points than the kernel's
-  // mask of near-degenerate ones has bits, stay with the other kernels.)
-  if (t->hexline_bytes == 0 || t->hexline_bytes > 16 * 1024 || (split && t->hexline_plane > 64) || (mask & tlg::kOutFacetNormals) || (split && o->tile != 16))
+  // (In split precision planes of more points than the kernel's mask of near-degenerate ones has bits stay with
+  // the other kernels.)
+  if (t->hexline_bytes == 0 || (split && t->hexline_plane > 64) || (mask & tlg::kOutFacetNormals) || (split && o->tile != 16))
     return TLG_ERR_UNSUPPORTED;
   tlg::HexLineArgs a;
   std::memset(&a, 0, sizeof(a));
@@ -1473,18 +1475,21 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
         t->poly_bytes = (uint32_t)align16(t->poly_points + prule.points.size() * sizeof(tlg::PolyNode));
         // Rules beyond 32 KiB are read from global memory, so that they do not cost resident CTAs.
         t->poly_staged = t->poly_bytes <= 32 * 1024 ? t->poly_bytes : t->poly_planes;
-        t->off_poly = (uint32_t)align16(host_bytes);
-        host_bytes = (size_t)t->off_poly + t->poly_bytes;
+        t->off_poly = align16(host_bytes);
+        host_bytes = t->off_poly + t->poly_bytes;
         if (df && td == 3) {
           t->polydf_points = (uint32_t)(prule.lines.size() * sizeof(tlg::PolyDfNode));
           t->polydf_bytes = (uint32_t)align16(t->polydf_points + prule.points.size() * sizeof(tlg::PolyDfNode));
-          t->off_polydf = (uint32_t)align16(host_bytes);
-          host_bytes = (size_t)t->off_polydf + t->polydf_bytes;
+          t->off_polydf = align16(host_bytes);
+          host_bytes = t->off_polydf + t->polydf_bytes;
         }
       }
     }
     // Hexahedra Q1-Q2 in f32 and split precision: the lattice, then the rule's planes, lines and points in f32.
-    if (dtype != TLG_F64 && cell == tlg::kHexahedron && degree <= 2 && npoints > 0) {
+    // (Rules whose section would cost resident CTAs stay with the other kernels: none is built.)
+    const int64_t hexline_most = 16 * 1024;
+    if (dtype != TLG_F64 && cell == tlg::kHexahedron && degree <= 2 && npoints > 0 &&
+        npoints * (int64_t)sizeof(tlg::PolyNodeF) <= hexline_most) {
       std::vector<double> s1, lt;
       if (sf_permutation(cell, degree, family, s1, lt, pstarts)) {
         prule = tlg::poly_rule(cell, degree, points, npoints);
@@ -1494,9 +1499,12 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
         t->poly_planes = (uint32_t)align16(pstarts.size() * 4);
         t->poly_lines = (uint32_t)(t->poly_planes + prule.planes.size() * sizeof(tlg::PolyNodeF));
         t->poly_points = (uint32_t)(t->poly_lines + prule.lines.size() * sizeof(tlg::PolyNodeF));
-        t->hexline_bytes = (uint32_t)(t->poly_points + prule.points.size() * sizeof(tlg::PolyNodeF));
-        t->off_poly = (uint32_t)align16(host_bytes);
-        host_bytes = (size_t)t->off_poly + t->hexline_bytes;
+        const int64_t bytes = t->poly_points + (int64_t)(prule.points.size() * sizeof(tlg::PolyNodeF));
+        if (bytes <= hexline_most) {
+          t->hexline_bytes = (uint32_t)bytes;
+          t->off_poly = align16(host_bytes);
+          host_bytes = t->off_poly + t->hexline_bytes;
+        }
       }
     }
     t->host.assign(host_bytes, 0);
