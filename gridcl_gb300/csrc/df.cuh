@@ -194,8 +194,9 @@ __device__ __forceinline__ double df_to_f64(float h, float l) {
   // and 1.5 * 2^23 + n is exact in [2^23, 2^24], its low mantissa bits n. The scale carries h's
   // sign, so that n is the change of h's magnitude.
   const float scale = __uint_as_float(((300u << 23) - (hb & 0x7F800000u)) | (hb & 0x80000000u));
-  const float t = __fmaf_rn(l, scaled ? scale : 0.0f, 12582912.0f);
-  const int n = (int)(__float_as_uint(t) - 0x4B400000u);
+  const float t = __fmaf_rn(l, scale, 12582912.0f);
+  // (The select is on n: an infinite or NaN h has a NaN tail, which a zero scale would let through.)
+  const int n = scaled ? (int)(__float_as_uint(t) - 0x4B400000u) : 0;
   // A power of two h whose magnitude l lowers lands in the binade below, whose ulp is half: the
   // same change of value is twice as many units of the mantissa field there.
   const int shift = 6 + (int)(((hb << 9) == 0u) & (n < 0));
