@@ -1461,8 +1461,8 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
         }
         if (!C.empty()) pstarts.push_back((uint32_t)pterms.size());
       }
-      if (!pstarts.empty()) {
-        prule = tlg::poly_rule(cell, degree, points, npoints);
+      if (!pstarts.empty()) prule = tlg::poly_rule(cell, degree, points, npoints);
+      if (!prule.points.empty()) {
         t->poly_nplanes = (int)prule.planes.size();
         t->poly_nlines = (int)prule.lines.size();
         for (const tlg::PolyNode& p : prule.planes) t->poly_plane_lines = std::max(t->poly_plane_lines, p.count);
@@ -1491,8 +1491,8 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
     if (dtype != TLG_F64 && cell == tlg::kHexahedron && degree <= 2 && npoints > 0 &&
         npoints * (int64_t)sizeof(tlg::PolyNodeF) <= hexline_most) {
       std::vector<double> s1, lt;
-      if (sf_permutation(cell, degree, family, s1, lt, pstarts)) {
-        prule = tlg::poly_rule(cell, degree, points, npoints);
+      if (sf_permutation(cell, degree, family, s1, lt, pstarts)) prule = tlg::poly_rule(cell, degree, points, npoints);
+      if (!prule.points.empty()) {
         t->poly_nplanes = (int)prule.planes.size();
         std::vector<int> of_plane(prule.planes.size(), 0);
         for (const tlg::PolyNode& l : prule.lines) t->hexline_plane = std::max(t->hexline_plane, of_plane[l.plane] += l.count);

@@ -91,6 +91,8 @@ std::vector<double> poly_expansion(int cell, int degree, const std::vector<doubl
 
 PolyRule poly_rule(int cell, int degree, const double* points, int64_t npoints) {
   const int td = tdim(cell);
+  for (int64_t i = 0; i < npoints * td; ++i)
+    if (!std::isfinite(points[i])) return {};
   // Planes by z, lines by (z, y), in order of first appearance.
   struct Line {
     double y;

@@ -40,7 +40,8 @@ enum PolyBasis { kCentred, kLine };
 std::vector<double> poly_expansion(int cell, int degree, const std::vector<double>& nodes, PolyBasis basis);
 
 // The point set in planes (equal z; one plane in 2D) of lines (equal y) of points, in order of
-// first appearance; lines of more than kPolyLine points in near-equal parts.
+// first appearance; lines of more than kPolyLine points in near-equal parts. Empty when a coordinate is
+// not finite: such a point shares no line (NaN has no order), and its values are the tabulation's.
 constexpr int kPolyLine = 4;
 struct PolyRule {
   std::vector<PolyNode> planes, lines, points;
