@@ -198,6 +198,9 @@ __global__ void __launch_bounds__(kEvalThreads, P == 1 ? 4 : 3) eval_hexline_ker
         }
       }
       u[0] = 0.0f;
+      // (A node that is not finite reaches every point, as in poly_coefficients.)
+      if (MID && (__float_as_uint(u[K - 1]) & 0x7F800000u) == 0x7F800000u)
+        u[0] = u[1] = u[N] = u[N * N] = __uint_as_float(0x7FC00000u);
 #pragma unroll
       for (int m = 0; m < K; ++m) xs[(m * 3 + g) * T] = u[m];
     }

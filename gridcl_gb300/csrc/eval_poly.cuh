@@ -142,12 +142,17 @@ __device__ __forceinline__ double poly_der_n(int deg, const double* A, const Pol
   return poly_der<P, AT_MID>(A, u);
 }
 
+// Whether v is infinite or NaN (an integer test: a comparison of doubles takes the FP64 pipe), and a NaN.
+__device__ __forceinline__ bool poly_bad(double v) { return (__double2hiint(v) & 0x7FF00000) == 0x7FF00000; }
+__device__ __forceinline__ double poly_nan() { return __hiloint2double(0x7FF80000, 0); }
+
 // The three stages of one item, each with its middle point's form: P_ab and Q_ab of a plane and
 // coordinate (strides between the coefficients of c and the sums of o), the line's A, D and E from
 // them, and X and J at a point.
 template <int CELL, int P, int STRIDE, bool AT_MID, int OSTRIDE = STRIDE>
 __device__ __forceinline__ void poly_plane(const double* c, const PolyAt& z, bool want_j, double* o) {
   using S = PolySpace<CELL, P>;
+  [[maybe_unused]] bool bad = false;
 #pragma unroll
   for (int b = 0; b <= P; ++b)
 #pragma unroll
@@ -158,7 +163,11 @@ __device__ __forceinline__ void poly_plane(const double* c, const PolyAt& z, boo
         if (l <= S::cc(x, b) && (!AT_MID || l < 2)) v[l] = c[S::ci(x, b, l) * STRIDE];
       o[S::pi(x, b) * OSTRIDE] = poly_val_n<P, AT_MID>(S::cc(x, b), v, z);
       if (want_j && S::cc(x, b) > 0) o[(S::AB + S::qi(x, b)) * OSTRIDE] = poly_der_n<P, AT_MID>(S::cc(x, b), v, z);
+      if constexpr (AT_MID && !S::kTensor) bad = bad || poly_bad(v[1]);
     }
+  // (Nodes of a prism's outer layers that are not finite, as poly_coefficients does for tensor cells.)
+  if constexpr (AT_MID && !S::kTensor)
+    if (bad) o[S::pi(0, 0) * OSTRIDE] = o[S::pi(1, 0) * OSTRIDE] = o[S::pi(0, 1) * OSTRIDE] = poly_nan();
 }
 
 template <int CELL, int P, int GD, int STRIDE, bool AT_MID>
@@ -267,6 +276,12 @@ __device__ __forceinline__ bool poly_coefficients(const PolyCells& a, int64_t c0
         }
       }
       u[0] = 0.0;
+      // A node that is not finite makes the whole coordinate so, as the Lagrange sums do (0 times NaN): at a
+      // middle point, which takes the low coefficients only, too. Every node is in the highest coefficient.
+      if (N == 3 && poly_bad(u[K - 1])) {
+        u[0] = u[1] = u[N] = poly_nan();
+        if constexpr (TD == 3) u[N * N] = poly_nan();
+      }
 #pragma unroll
       for (int m = 0; m < K; ++m) cs[m * (GD * W) + i] = u[m];
     }
