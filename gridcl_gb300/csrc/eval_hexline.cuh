@@ -131,7 +131,9 @@ __global__ void __launch_bounds__(kEvalThreads, P == 1 ? 4 : 3) eval_hexline_ker
   const NT* nodes = static_cast<const NT*>(a.nodes);
   const uint32_t mask = a.mask;
   const int nq = a.num_points, shift = SHIFT >= 0 ? SHIFT : a.tile_shift;
-  const float lim = fminf(9.0f * a.cond_limit * a.cond_limit, 3.402823466e38f);
+  // (An infinite limit leaves NaN only above it.)
+  const float lim = a.cond_limit <= 3.402823466e38f ? fminf(9.0f * a.cond_limit * a.cond_limit, 3.402823466e38f)
+                                                    : a.cond_limit;
 
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < a.padded; c += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t* row = a.dofmap + min(a.first_cell + c, a.last_cell) * K;
