@@ -15,13 +15,18 @@
 // per SM, issue 31 % active, 3.04 ms on the P2 tetrahedra below.)
 //
 // X adds the cell's offset in FP64. f64 bit patterns are assembled by df_to_f64_fast, ten integer
-// operations and an FFMA; values it does not take (zero mantissas, magnitudes outside [2^-81, 2^127),
-// NaN) send the thread's field through df_to_f64.
+// operations and an FFMA; it does not take zero mantissas, magnitudes outside [2^-81, 2^127) and NaN. Zeros and
+// powers of two, which axis-aligned and straight cells have at every point, are mended in place (df_mend);
+// the others send three components of the thread's field through df_to_f64 out of line. J leaves three
+// components at a time as K does: nine at a time with the mending spilled. Q2 hexahedra, 140,608 cells at 27
+// points, axis-aligned / curved, all four factors: 0.69 / 0.41 ms when every special value went out of line,
+// 0.485 / 0.408 so (three lanes per cell: 0.50 either way); mending every value without a branch cost the
+// curved cells 8 %.
 //
 // Bound by the issue slots (50 % of them used at 16 warps per SM: dependent double-float chains, and 80-90 %
 // hits in the instruction cache) with the FP64 pipe 38 % and the integer pipe 37 % active. GB300, x, J, det J
 // and K, ms, the former kernels (one thread or three lanes per cell) -> this one: P2 tetrahedra, 1,572,864
-// cells at 24 points 3.04 -> 1.96; Q2 hexahedra, 500,000 at 27 points 1.74 -> 1.38; P3 tetrahedra, 180,000 at
+// cells at 24 points 3.04 -> 1.91; Q2 hexahedra, 500,000 at 27 points 1.74 -> 1.38; P3 tetrahedra, 180,000 at
 // 64 points 2.36 -> 0.88; 1,000 P2 tetrahedra at 27 points 0.073 -> 0.032 (the host's call).
 #pragma once
 
@@ -82,16 +87,25 @@ __device__ __forceinline__ double df_to_f64_fast(float h, float l, bool& special
   return __longlong_as_double((long long)bits);
 }
 
+// df_to_f64_fast's value d of (h, l) mended where h is a zero or a power of two in range, which axis-aligned
+// and straight cells have everywhere; `rest` is set for the other special values.
+__device__ __forceinline__ void df_mend(float h, double& d, bool& rest) {
+  const uint32_t hb = __float_as_uint(h), mag = hb << 1;
+  rest = rest || (mag != 0u && mag - (46u << 24) >= (208u << 24));
+  // 64 n, d's low word as h's mantissa is zero: a power of two whose magnitude l lowers lands in the binade
+  // below, whose ulp is half.
+  const int n6 = __double2loint(d);
+  if ((hb << 9) == 0u && n6 < 0) d = __longlong_as_double(__double_as_longlong(d) + n6);
+  if (mag == 0u) d = __hiloint2double((int)hb, 0);
+}
+
 using Dp = DF<float2>;
 
 // The n entries (h0, h1, l0, l1) of t as the two f64 (hi, lo words), in place; out of line, as it would
-// double the kernel's code for values that are rarely special.
+// double the kernel's code for values that are rare (tiny, huge, not finite).
 static __device__ __noinline__ void df_pairs_slow(float4* t, int n) {
   for (int c = 0; c < n; ++c) {
-    // (An infinite or NaN head has a NaN tail: left out.)
-    const float lx = (__float_as_uint(t[c].x) << 1) >= 0xFF000000u ? 0.0f : t[c].z;
-    const float ly = (__float_as_uint(t[c].y) << 1) >= 0xFF000000u ? 0.0f : t[c].w;
-    const double x = df_to_f64(t[c].x, lx), y = df_to_f64(t[c].y, ly);
+    const double x = df_to_f64(t[c].x, t[c].z), y = df_to_f64(t[c].y, t[c].w);
     t[c] = make_float4(__int_as_float(__double2hiint(x)), __int_as_float(__double2loint(x)),
                        __int_as_float(__double2hiint(y)), __int_as_float(__double2loint(y)));
   }
@@ -106,15 +120,23 @@ __device__ __forceinline__ void df_pair_to_f64(const Dp* v, double2* d) {
     d[c].x = df_to_f64_fast(v[c].h.x, v[c].l.x, special);
     d[c].y = df_to_f64_fast(v[c].h.y, v[c].l.y, special);
   }
-  if (special) {
-    float4 t[LEN];
-#pragma unroll
-    for (int c = 0; c < LEN; ++c) t[c] = make_float4(v[c].h.x, v[c].h.y, v[c].l.x, v[c].l.y);
-    df_pairs_slow(t, LEN);
+  if (__builtin_expect(special, 0)) {
+    bool rest = false;
 #pragma unroll
     for (int c = 0; c < LEN; ++c) {
-      d[c].x = __hiloint2double(__float_as_int(t[c].x), __float_as_int(t[c].y));
-      d[c].y = __hiloint2double(__float_as_int(t[c].z), __float_as_int(t[c].w));
+      df_mend(v[c].h.x, d[c].x, rest);
+      df_mend(v[c].h.y, d[c].y, rest);
+    }
+    if (__builtin_expect(rest, 0)) {
+      float4 t[LEN];
+#pragma unroll
+      for (int c = 0; c < LEN; ++c) t[c] = make_float4(v[c].h.x, v[c].h.y, v[c].l.x, v[c].l.y);
+      df_pairs_slow(t, LEN);
+#pragma unroll
+      for (int c = 0; c < LEN; ++c) {
+        d[c].x = __hiloint2double(__float_as_int(t[c].x), __float_as_int(t[c].y));
+        d[c].y = __hiloint2double(__float_as_int(t[c].z), __float_as_int(t[c].w));
+      }
     }
   }
 }
@@ -276,7 +298,15 @@ __global__ void __launch_bounds__(128, 4) eval_dfpoly_kernel(const __grid_consta
         float h, l;
         bool special = false;
         df_split_int(v[m], h, l, special);
-        if (special) df_split(v[m], h, l);
+        if (__builtin_expect(special, 0)) {
+          const int hi = __double2hiint(v[m]);
+          if (((hi << 1) | __double2loint(v[m])) == 0) {  // zero
+            h = __int_as_float(hi);
+            l = 0.0f;
+          } else {
+            df_split(v[m], h, l);
+          }
+        }
         o[m * (ROW * 4)] = h;
         o[m * (ROW * 4) + 2] = l;
       }
@@ -332,7 +362,12 @@ __global__ void __launch_bounds__(128, 4) eval_dfpoly_kernel(const __grid_consta
           df_store_pair<3>(a.out[0] + q * 48 + l16, d, wide);
         }
         if (!want_j) continue;
-        if (mask & kOutJacobian) df_put_pair<9>(a.out[1] + q * 144 + l16, j, wide);
+        if (mask & kOutJacobian) {
+          double* pj = a.out[1] + q * 144 + l16;
+          df_put_pair<3>(pj, j, wide);
+          df_put_pair<3>(pj + 48, j + 3, wide);
+          df_put_pair<3>(pj + 96, j + 6, wide);
+        }
         if (!(mask & (kOutDetJ | kOutPinv))) continue;
         // Row 0 of the cofactors gives det J; K leaves three entries (a component g) at a time.
         Dp r0[3];
