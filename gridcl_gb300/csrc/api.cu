@@ -2637,6 +2637,14 @@ tlg_status tlg_batch_tune(tlg_batch* b, void* stream, int* grids) {
   // rows per thread; cooperative: four lanes per cell; tcgen05: 64-cell tiles by 8-point chunks).
   int fixed = TLG_STRATEGY_AUTO;
   if (!wanted_strategy(TLG_FAMILY_JACOBIAN, &fixed)) return finish(TLG_ERR_INVALID_ARGUMENT);
+  // Blocks whose kernel has one grid for its cells (the polynomial kernels) have no grid to choose.
+  std::vector<char> takes_grid(b->tables.size(), 0);
+  auto probe_grid = [&](size_t i) -> tlg_status {
+    tlg::g_grid_taken = false;
+    const tlg_status st = eval_with_grid(b, i, s, sms);
+    takes_grid[i] = tlg::g_grid_taken ? 1 : 0;
+    return st;
+  };
   bool caller_fixed = fixed != TLG_STRATEGY_AUTO;
   for (int f = 0; f < kFamilies; ++f) caller_fixed = caller_fixed || g_override[f] >= 0;
   for (size_t i = 0; i < b->tables.size(); ++i) {
@@ -2670,8 +2678,10 @@ tlg_status tlg_batch_tune(tlg_batch* b, void* stream, int* grids) {
       }
       b->strategy[i] = strat;
       int mult = 0;
+      const tlg_status probed = probe_grid(i);
+      if (probed != TLG_OK) return finish(probed);
       for (int c : cands) {
-        if (c == 0) continue;  // timed above
+        if (c == 0 || !takes_grid[i]) continue;  // (0: timed above)
         const int grid = c * sms;
         float ms = 0.0f;
         tlg_status st = median_ms([&] { return eval_with_grid(b, i, s, grid); }, &ms);
@@ -2687,7 +2697,9 @@ tlg_status tlg_batch_tune(tlg_batch* b, void* stream, int* grids) {
       g_tune_cache[key] = choice;
     }
     b->strategy[i] = choice.first;
-    b->grid[i] = choice.second == 0 ? 0 : choice.second * sms;
+    const tlg_status probed = probe_grid(i);
+    if (probed != TLG_OK) return finish(probed);
+    b->grid[i] = choice.second == 0 || !takes_grid[i] ? 0 : choice.second * sms;
   }
   // Joint pass: the graph runs the blocks concurrently (or in turn), so each block's best grid
   // alone is only the start. Every comparison times the whole graph (time_graph), and a change
@@ -2729,7 +2741,7 @@ tlg_status tlg_batch_tune(tlg_batch* b, void* stream, int* grids) {
     return st;
   };
   if (joint.size() == b->tables.size() + 1) {
-    for (size_t i = 0; i < b->tables.size(); ++i) b->grid[i] = joint[i];
+    for (size_t i = 0; i < b->tables.size(); ++i) b->grid[i] = takes_grid[i] ? joint[i] : 0;
     b->serial = joint.back() != 0;
   } else if (b->tables.size() > 1) {
     float serial_ms = 0.0f, par_ms = 0.0f, serial_max = 0.0f, par_max = 0.0f, best = 0.0f;
@@ -2748,7 +2760,7 @@ tlg_status tlg_batch_tune(tlg_batch* b, void* stream, int* grids) {
       int chosen = keep;
       for (int c : cands) {
         const int grid = c == 0 ? 0 : c * sms;
-        if (grid == keep) continue;
+        if (grid == keep || !takes_grid[i]) continue;
         b->grid[i] = grid;
         float ms = 0.0f;
         st = time_graph(&ms);

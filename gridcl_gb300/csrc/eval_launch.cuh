@@ -10,11 +10,14 @@ namespace tlg {
 
 // A grid size chosen by the batch autotuner for the next launches on this thread (0: none).
 inline thread_local int g_grid_override = 0;
+// Set by launches on this thread whose grid that choice is (the autotuner clears and reads it).
+inline thread_local bool g_grid_taken = false;
 
 // Grid of persistent CTAs: enough to cover the range, at most the resident CTAs of the device
 // (or the autotuner's choice).
 template <typename Kernel>
 inline int persistent_grid(Kernel kern, size_t smem, int64_t work_items, int threads) {
+  g_grid_taken = true;
   if (g_grid_override > 0) return g_grid_override;
   static thread_local int sms = 0;
   if (sms == 0) {
