@@ -545,6 +545,59 @@ tlg_status eval_poly(const tlg_tables* t, const tlg_block* b, const tlg_outputs*
   return ok();
 }
 
+// FP64 operations of the polynomial kernels per plane, line and point and coordinate: the sums' multiply-adds
+// of the points alone, and with J (eval_poly.cuh).
+struct PolyOps {
+  int plane, line, point;
+};
+PolyOps poly_ops(int cell, int p, bool want_x, bool want_j) {
+  const bool tri = cell == tlg::kTriangle || cell == tlg::kTetrahedron || cell == tlg::kPrism;
+  const bool tet = cell == tlg::kTetrahedron, volume = tlg::tdim(cell) == 3;
+  auto der = [](int d) { return d == 3 ? 4 : d == 2 ? 1 : 0; };  // (a value of degree d: d)
+  PolyOps n = {0, 0, 0};
+  for (int b = 0; b <= p && volume; ++b)
+    for (int a = 0; a <= (tri ? p - b : p); ++a) {
+      const int c = tet ? p - a - b : p;
+      n.plane += c + (want_j ? der(c) : 0);
+    }
+  const int da = tri ? p - 1 : p, ea = tet ? p - 1 : p;
+  for (int a = 0; a <= p; ++a) n.line += (tri ? p - a : p) + (a <= da ? der(tri ? p - a : p) : 0);
+  for (int a = 0; a <= ea && volume && want_j; ++a) n.line += tet ? p - 1 - a : tri ? p - a : p;
+  n.point = (want_x ? p + 1 : 0) + (want_j ? der(p) + da + (volume ? ea : 0) : 0);
+  return n;
+}
+
+// Whether f64 cells with both kernels run the polynomial one rather than eval_direct_kernel, which one thread
+// per cell runs over its points. In FP64 operations per cell of a device that does them at full rate: that one
+// takes its Lagrange sums and its factors at every point, on the SMs that CTAs of 128 cells reach; this one
+// its planes', lines' and points' sums, the factors (once per line where J is constant), and a start (gather,
+// coefficients, barriers) of 12 operations per node and coordinate on simplices, 9 on prisms, 6 on tensor
+// cells, and of two microseconds at least. The starts are fitted to 1,200 timings of both kernels (rules of 1
+// to 27 points, scattered and collapsed, five sets of factors, 3,000 and 128,000 to 320,000 cells); the
+// choice is on average within 1.2 % of the faster. GB300, ms, direct / polynomial, 280,000 P2 tetrahedra: one
+// point, four factors 0.088 / 0.194, det J alone 0.052 / 0.168, points alone 0.022 / 0.153; 2 x 2 x 2 points, four
+// factors 0.67 / 0.36, points alone 0.136 / 0.194. Blocks below 64 cells per SM always run the polynomial kernel:
+// the two differ by a few microseconds there, and results do not depend on the factors asked for. (By the
+// block's cells, so that ranges of a block agree; at tiles other than 16 the loops kernel, which has the
+// direct kernel's bits, takes its place.)
+bool poly_preferred(const tlg_tables* t, const tlg_block* b, uint32_t mask) {
+  if (!t->staged || b->num_cells < (int64_t)64 * 152) return true;
+  const bool want_x = (mask & tlg::kOutPoints) != 0, want_j = (mask & ~tlg::kOutPoints) != 0;
+  const bool want_k = (mask & (tlg::kOutPinv | tlg::kOutFacetNormals)) != 0;
+  const bool want_d = (mask & (tlg::kOutDetJ | tlg::kOutNormals)) != 0;
+  const bool surface = t->td < t->gd, affine = t->degree == 1 && (t->cell == tlg::kTriangle || t->cell == tlg::kTetrahedron);
+  const double factors = (want_d ? (surface ? 45 : t->td == 3 ? 14 : 3) : 0) + (want_k ? (surface ? 70 : t->td == 3 ? 40 : 16) : 0);
+  const double q = (double)t->q, nodes = (double)t->k * t->gd, cells = (double)b->num_cells;
+  const double reach = std::min(1.0, std::ceil(cells / 128) / 152);
+  const double direct = q * (nodes * ((want_x ? 1 : 0) + (want_j ? t->td : 0)) + factors) / reach;
+  const PolyOps n = poly_ops(t->cell, t->degree, want_x, want_j);
+  const bool simplex = t->cell == tlg::kTriangle || t->cell == tlg::kTetrahedron;
+  const double start = (simplex ? 12 : t->cell == tlg::kPrism ? 9 : 6) * nodes;
+  const double poly = std::max(start, 1.2e6 / cells) + (affine ? t->poly_nlines : q) * factors +
+                      t->gd * ((double)t->poly_nplanes * n.plane + (double)t->poly_nlines * n.line + q * n.point);
+  return direct >= 0.9 * poly;
+}
+
 // The FP32 line kernel of hexahedra (f32 meshes at any tile, split precision at tile 16; no facet normals);
 // `found` is false where it does not apply.
 tlg_status eval_hexline(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o, uint32_t mask,
@@ -1779,7 +1832,11 @@ tlg_status eval_dispatch(const tlg_tables* t, const tlg_block* b, const tlg_outp
   const bool is_auto = strategy == TLG_STRATEGY_AUTO;
   // f64 and double-float cells with a polynomial kernel: it is the sum factorisation of tensor rules
   // (recorded so) and the direct kernel of the others.
-  if (t->poly_bytes > 0 && (is_auto || strategy == TLG_STRATEGY_DIRECT || (strategy == TLG_STRATEGY_SUMFACT && t->sf_ok))) {
+  // (Under AUTO and DIRECT the f64 calls that poly_preferred declines go on to the direct kernel.)
+  const bool sumfact = strategy == TLG_STRATEGY_SUMFACT && t->sf_ok;
+  const bool poly = t->poly_bytes > 0 && (sumfact || ((is_auto || strategy == TLG_STRATEGY_DIRECT) &&
+                                                      (t->df || poly_preferred(t, b, mask))));
+  if (poly) {
     bool found = false;
     const int ran = t->sf_ok && strategy != TLG_STRATEGY_DIRECT ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT;
     tlg_status st = t->df ? eval_dfpoly(t, b, o, mask, ran, s, &found) : eval_poly(t, b, o, mask, ran, s, &found);

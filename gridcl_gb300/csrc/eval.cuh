@@ -26,7 +26,8 @@
 //    f32 fields, and an FP64 recompute of J, det J and K at points whose condition estimate
 //    exceeds a limit (counted in a device counter).
 //  - eval_direct_kernel<F, TD, GD, K, TILE>: scalar, everything unrolled (f64 intervals, pyramids P1-P3, P4
-//    triangles; the other f64 elements run the polynomial kernel of eval_poly.cuh).
+//    triangles; the other f64 elements at few points or for points alone, else the polynomial kernel of
+//    eval_poly.cuh).
 //  - eval_loops_kernel<F, TD, GD>: K and the tile at run time (every other element and tile).
 // Hexahedra on f32 meshes and in split precision run the line kernel of eval_hexline.cuh.
 #pragma once

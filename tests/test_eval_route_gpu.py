@@ -1,0 +1,53 @@
+"""f64 evaluation at few points, or of points alone, on meshes that fill the device: the unrolled kernel runs
+(bit for bit the loops kernel's values), for every cell that has it; rules of shared lines and small meshes
+keep the polynomial kernel. Both agree to rounding."""
+
+import numpy as np
+import pytest
+import torch
+
+import gridcl_gb300 as tg
+from gridcl_gb300 import meshes
+
+pytestmark = pytest.mark.gpu
+
+ALL = ("points", "jacobian", "detj", "pinv")
+CELLS = [("Tetrahedron", 1, 3), ("Tetrahedron", 2, 3), ("Tetrahedron", 3, 3), ("Hexahedron", 1, 3),
+         ("Hexahedron", 2, 3), ("Prism", 1, 3), ("Prism", 2, 3), ("Triangle", 1, 2), ("Triangle", 2, 3),
+         ("Triangle", 3, 2), ("Quadrilateral", 1, 3), ("Quadrilateral", 2, 2)]
+
+
+def mesh_of(cell, degree, gd):
+    if gd == 2 or cell in ("Triangle", "Quadrilateral"):
+        m = meshes.square_box(cell, 100 if cell == "Triangle" else 140, degree)
+        m.nodes = meshes.jitter_interior(m.nodes, m.nodes, 0.0005, 2026)
+        return m if gd == 2 else meshes.HostMesh(3, np.concatenate([m.nodes, 0.1 * np.sin(3.0 * m.nodes[:, :1])], 1),
+                                                 m.blocks)
+    return meshes.curved_box(cell, {"Tetrahedron": 15, "Hexahedron": 27, "Prism": 22}[cell], degree, jitter=0.001)
+
+
+def run(g, ps, names, strategy="auto"):
+    with tg.with_strategy(strategy):
+        return {f: v.to_host_cell_major() for f, v in tg.geometric_factors_block(g, 0, ps, names).items()}
+
+
+@pytest.mark.parametrize("cell,degree,gd", CELLS)
+def test_few_points(cuda, cell, degree, gd):
+    td = tg.refcell.tdim(cell)
+    mesh = mesh_of(cell, degree, gd)
+    assert mesh.blocks[0].num_cells >= 128 * 152
+    g = tg.Geometry.from_host(mesh, dtype=torch.float64)
+    scattered = np.random.default_rng(3).uniform(0.05, 0.3, size=(3, td))
+    for pts, names in ((scattered[:1], ALL), (scattered[:1], ("detj",)), (scattered, ("points",))):
+        ps = tg.PointSet(cell, pts, np.ones(len(pts)))
+        got, want = run(g, ps, names), run(g, ps, names, "loops")
+        for f in names:
+            assert np.array_equal(got[f], want[f]), (f, len(pts))
+        tile4 = tg.geometric_factors_block(g, 0, ps, names, tile=4, max_chunk_cells=5000)
+        assert np.array_equal(tile4[names[0]].to_host_cell_major(), got[names[0]])
+    pts, w = tg.refcell.collapsed_rule(cell, (4, 4, 3)[:td])
+    ps = tg.PointSet(cell, pts, w)
+    got, want = run(g, ps, ALL), run(g, ps, ALL, "loops")
+    for f in ALL[:3]:  # (K is the condition number times further off, and jittered P3 triangles reach 1e5)
+        assert np.abs(got[f] - want[f]).max() <= 1e-11 * np.abs(want[f]).max(), f
+    assert not np.array_equal(got["detj"], want["detj"])  # the polynomial kernel's rounding
