@@ -641,6 +641,52 @@ tlg_status eval_hexline(const tlg_tables* t, const tlg_block* b, const tlg_outpu
   return ok();
 }
 
+// Whether double-float cells run the polynomial kernel rather than the kernels they had before it (eval_df_kernel
+// on tetrahedra and on points without tensor structure, the sum factorisations on the others). That one
+// pays where lines and planes are shared: on points of their own planes every point costs a plane's FP64 sums
+// and their splits. Tetrahedra and prisms: both sides as picoseconds per cell on a full device, fitted to 240 and
+// 160 timings (the rules and factors of poly_preferred): per node and coordinate, plane sum, FP64 operation of
+// a plane, of a line, of a point, value stored and K; there per node and coordinate, double-float term,
+// value, det J and K. The polynomial kernel, the more accurate, is left where the others take 0.8 of its time by
+// this count; on part of the device the one-cell-per-thread kernels leave SMs idle, so 0.65 below 256 cells per
+// SM, 0.35 (prisms 0.55) below 64. On average within 1 to 2.5 % of the faster. GB300, ms, former kernels / polynomial, 280,000 P2 tetrahedra: 4 x 3 x 2 points, four
+// factors 0.51 / 0.35, det J alone 0.198 / 0.201; 24 scattered points, four factors 0.51 / 1.33; 140,000 Q2
+// hexahedra, 3 x 3 x 3 points 0.50 / 0.41, 2 x 2 x 2 0.22 / 0.24, 14 scattered 0.45 / 1.10.
+bool dfpoly_preferred(const tlg_tables* t, const tlg_block* b, uint32_t mask) {
+  const bool rows = t->staged && t->dfrows_bytes > 0 &&
+                    (size_t)(t->bytes + 15) / 16 * 16 + tlg::df_slot_bytes((int)t->k, t->gd, t->df_mono) <= (size_t)227 * 1024;
+  if (!t->sf_ok && !rows) return true;  // no other double-float kernel
+  const bool small = b->num_cells < (int64_t)64 * 152;
+  const double q = (double)t->q, planes = t->poly_nplanes, lines = t->poly_nlines;
+  if (t->cell == tlg::kHexahedron) {  // lines of two points at Q1, three at Q2
+    if (small && t->degree == 1) return true;
+    return t->degree == 1 ? q >= 4 && q >= 2 * lines : q >= 9 && q >= 3 * lines;
+  }
+  const bool tet = t->cell == tlg::kTetrahedron;
+  const bool want_x = (mask & tlg::kOutPoints) != 0, want_j = (mask & ~tlg::kOutPoints) != 0;
+  const bool det = (mask & tlg::kOutDetJ) != 0, pinv = (mask & tlg::kOutPinv) != 0;
+  const double values = (want_x ? 3 : 0) + (mask & tlg::kOutJacobian ? 9 : 0) + (det ? 1 : 0) + (pinv ? 9 : 0);
+  const int p = t->degree, n = p + 1, tri = n * (n + 1) / 2;
+  const int k = (int)t->k, plane = tri + (want_j ? (tet ? p * n / 2 : tri) : 0);
+  const PolyOps ops = poly_ops(t->cell, p, want_x, want_j);
+  const double nodes = 3.0 * k, sums = 3 * planes * plane, fp_plane = 3 * planes * ops.plane, fp_line = 3 * lines * ops.line,
+               fp_point = 3 * q * ops.point;
+  double poly, other;
+  if (tet) {
+    const double even = (double)((t->q + 1) / 2 * 2);  // its kernel works on pairs of points
+    const int terms = (want_x ? k - 1 : 0) + (want_j ? p * n * (n + 1) / 2 : 0);
+    poly = 15.1 * nodes + 0.76 * sums + 4.4 * fp_plane + 0.22 * fp_line + 0.21 * fp_point +
+           q * (1.2 * values + (pinv ? 5.7 : 0));
+    other = 6.6 * nodes + even * (0.74 * 3 * terms + 0.72 * values + (det ? 0.4 : 0) + (pinv ? 11.9 : 0));
+  } else {
+    const double terms = t->sf_ok ? 3 * (q / planes * n * tri * 3 + q * n * 4) : 3 * q * k * ((want_x ? 1 : 0) + (want_j ? 3 : 0));
+    poly = 10.4 * nodes + 0.94 * sums + 2.8 * fp_plane + 3.8 * fp_line + 0.77 * fp_point +
+           q * (0.86 * values + (pinv ? 8.3 : 0));
+    other = 5.75 * nodes + 0.43 * terms + q * (1.2 * values + (det ? 1.9 : 0) + (pinv ? 12.3 : 0));
+  }
+  return other >= (small ? tet ? 0.35 : 0.55 : b->num_cells < (int64_t)256 * 152 ? 0.65 : 0.8) * poly;
+}
+
 // The double-float polynomial kernel (TLG_DF64 tables of volume cells, tile 16, no facet normals);
 // `found` is false where none is compiled for the tables.
 tlg_status eval_dfpoly(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o, uint32_t mask, int family,
@@ -1832,10 +1878,12 @@ tlg_status eval_dispatch(const tlg_tables* t, const tlg_block* b, const tlg_outp
   const bool is_auto = strategy == TLG_STRATEGY_AUTO;
   // f64 and double-float cells with a polynomial kernel: it is the sum factorisation of tensor rules
   // (recorded so) and the direct kernel of the others.
-  // (Under AUTO and DIRECT the f64 calls that poly_preferred declines go on to the direct kernel.)
+  // (Calls that poly_preferred and dfpoly_preferred decline go on to the kernels below; f64 has no other sum
+  // factorisation of these cells.)
   const bool sumfact = strategy == TLG_STRATEGY_SUMFACT && t->sf_ok;
-  const bool poly = t->poly_bytes > 0 && (sumfact || ((is_auto || strategy == TLG_STRATEGY_DIRECT) &&
-                                                      (t->df || poly_preferred(t, b, mask))));
+  const bool poly = t->poly_bytes > 0 && (is_auto || strategy == TLG_STRATEGY_DIRECT || sumfact) &&
+                    (t->df && o->tile == 16 ? dfpoly_preferred(t, b, mask)
+                                            : t->df || sumfact || poly_preferred(t, b, mask));
   if (poly) {
     bool found = false;
     const int ran = t->sf_ok && strategy != TLG_STRATEGY_DIRECT ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT;

@@ -13,7 +13,8 @@
 // is assembled into its f64 (df_to_f64) and stored into its QuadField chunk.
 //
 // What reaches it: surfaces, planar cells and pyramids; of tetrahedra, hexahedra and prisms the
-// calls that ask for facet normals (the others run the polynomial kernel of eval_dfpoly.cuh).
+// calls that ask for facet normals and those of few shared lines (dfpoly_preferred; the others run the
+// polynomial kernel of eval_dfpoly.cuh).
 #pragma once
 
 #include <cstdint>

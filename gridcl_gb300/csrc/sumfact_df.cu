@@ -1,6 +1,6 @@
 // Instantiations of the double-float sum-factorised kernels (sumfact_df.cuh): hexahedra Q1-Q3,
 // quadrilaterals Q1-Q5 (planar and embedded in 3D), prisms P1-P3, with and without facet normals,
-// and the three-lanes-per-cell Q3 hexahedra.
+// and the three-lanes-per-cell hexahedra.
 #include "eval_launch.cuh"
 #include "sumfact_df.cuh"
 
@@ -47,7 +47,11 @@ cudaError_t launch_sumfact_df3(int n, const SfArgs& a, size_t smem, cudaStream_t
   *found = true;
   // Ten cells per warp: the persistent grid covers padded / 10 warps.
   const int64_t work = (a.padded + 9) / 10 * 32;
-  // (Q1 and Q2 run the polynomial kernel of eval_dfpoly.cuh.)
+  // Register caps: three CTAs per SM at Q2 (168 registers; 220 without a cap ran 8.26 ms against
+  // 7.34 ms on 128^3 Q2 hexahedra, 128 registers 7.27 ms with 276 bytes of spills). Q1 and Q2: the rules
+  // that dfpoly_preferred leaves.
+  if (n == 2) return launch_persistent(sumfact_df3_kernel<2, 3>, a, work, smem, s);
+  if (n == 3) return launch_persistent(sumfact_df3_kernel<3, 3>, a, work, smem, s);
   if (n == 4) return launch_persistent(sumfact_df3_kernel<4, 2>, a, work, smem, s);
   *found = false;
   return cudaSuccess;

@@ -11,10 +11,11 @@
 // each pair's det J, K, normals and facet normals follow in double-float, assembled into f64 and
 // stored.
 //  - sumfact_df_kernel: one cell per thread (quadrilaterals, facet normals);
-//  - sumfact_df3_kernel: Q3 hexahedra with three lanes per cell, lane g computing coordinate g;
+//  - sumfact_df3_kernel: hexahedra with three lanes per cell, lane g computing coordinate g;
 //  - sumfact_prism_df_kernel: prisms, one cell per thread, the z points two at a time (rules with
 //    one line of points per plane, P3, facet normals).
-// Hexahedra Q1-Q2 and the other prisms run the polynomial kernel of eval_dfpoly.cuh.
+// Hexahedra Q1-Q2 and prisms P1-P2 run the polynomial kernel of eval_dfpoly.cuh where dfpoly_preferred
+// takes it.
 #pragma once
 
 #include <cstdint>

@@ -51,3 +51,37 @@ def test_few_points(cuda, cell, degree, gd):
     for f in ALL[:3]:  # (K is the condition number times further off, and jittered P3 triangles reach 1e5)
         assert np.abs(got[f] - want[f]).max() <= 1e-11 * np.abs(want[f]).max(), f
     assert not np.array_equal(got["detj"], want["detj"])  # the polynomial kernel's rounding
+
+
+def ms(g, ps, names, precision):
+    out = tg.geometric_factors_block(g, 0, ps, names, precision=precision)
+    times = []
+    for _ in range(7):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(5):
+            tg.geometric_factors_block(g, 0, ps, names, precision=precision, out=out)
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b))
+    return sorted(times)[3]
+
+
+@pytest.mark.parametrize("cell,degree,npts", [("Tetrahedron", 2, 24), ("Tetrahedron", 3, 14), ("Hexahedron", 2, 14),
+                                              ("Prism", 2, 14)])
+def test_double_float_at_scattered_points(cuda, cell, degree, npts):
+    """Points that share no line: the double-float path keeps its margin over f64 (0.3 to 0.5 of its time
+    measured; the polynomial kernel, whose planes' sums are in FP64, takes longer than f64 there), and its
+    error (3e-13 of the largest value)."""
+    n = {"Tetrahedron": 28, "Hexahedron": 51, "Prism": 40}[cell]  # 128,000 cells: the device is full
+    mesh = meshes.curved_box(cell, n, degree, jitter=0.02 / n)
+    g = tg.Geometry.from_host(mesh, dtype=torch.float64)
+    pts = np.random.default_rng(3).uniform(0.05, 0.3, size=(npts, 3))
+    ps = tg.PointSet(cell, pts, np.ones(npts))
+    for names in (ALL, ("detj",), ("points",)):
+        got = tg.geometric_factors_block(g, 0, ps, names, precision="df64")
+        want = tg.geometric_factors_block(g, 0, ps, names)
+        for f in names:
+            a, b = got[f].to_host_cell_major(), want[f].to_host_cell_major()
+            assert np.abs(a - b).max() <= 3e-13 * np.abs(b).max(), f
+    assert ms(g, ps, ALL, "df64") <= 0.8 * ms(g, ps, ALL, "native")
