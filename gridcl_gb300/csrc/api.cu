@@ -114,6 +114,7 @@ struct tlg_tables {
   // The section of f32 and split hexahedra Q1-Q2 in its place (eval_hexline.cuh).
   uint32_t hexline_bytes = 0;
   int hexline_plane = 0;  // the most points of a plane
+  int64_t hexline_lines = 0;
   // Double-float tables: the rule's lines and points as PolyDfNode.
   uint64_t off_polydf = 0;
   uint32_t polydf_bytes = 0, polydf_points = 0;
@@ -596,6 +597,20 @@ bool poly_preferred(const tlg_tables* t, const tlg_block* b, uint32_t mask) {
   const double poly = std::max(start, 1.2e6 / cells) + (affine ? t->poly_nlines : q) * factors +
                       t->gd * ((double)t->poly_nplanes * n.plane + (double)t->poly_nlines * n.line + q * n.point);
   return direct >= 0.9 * poly;
+}
+
+// Whether hexahedra on f32 meshes and in split precision run the line kernel rather than the paired one (at other
+// tiles the loops kernel): where J is wanted and lines have two or three points, of eight or six and more. On
+// points of their own lines every point costs a line, and points alone need J's sums of neither. Q1 with a cell
+// measure stays with the paired kernel, which sums it as it goes. GB300, 140,608 cells, us, paired / line, f32: Q2,
+// 3 x 3 x 3 points, four factors 87 / 78, points alone 32 / 37; 27 scattered points 87 / 94, points alone 31 / 73;
+// 2 x 1 x 1 points 23 / 29; split: 3 x 3 x 3 114 / 111, 27 scattered 113 / 131; Q1, 2 x 2 x 2, four factors with the
+// measure f32 20 / 23, split 35 / 37 (two kernels). Points alone on blocks below 64 cells per SM keep the line
+// kernel, so that results do not depend on the factors asked for there.
+bool hexline_preferred(const tlg_tables* t, const tlg_block* b, const tlg_outputs* o, uint32_t mask) {
+  if (!(mask & ~tlg::kOutPoints) && b->num_cells >= (int64_t)64 * 152) return false;
+  if (o->cell_measure && t->degree == 1) return false;
+  return (t->q >= 8 && t->q >= 2 * t->hexline_lines) || (t->q >= 6 && t->q >= 3 * t->hexline_lines);
 }
 
 // The FP32 line kernel of hexahedra (f32 meshes at any tile, split precision at tile 16; no facet normals);
@@ -1593,6 +1608,7 @@ tlg_status tlg_tables_create(int cell, int degree, int family, int gdim, int dty
       if (sf_permutation(cell, degree, family, s1, lt, pstarts)) prule = tlg::poly_rule(cell, degree, points, npoints);
       if (!prule.points.empty()) {
         t->poly_nplanes = (int)prule.planes.size();
+        t->hexline_lines = (int64_t)prule.lines.size();
         std::vector<int> of_plane(prule.planes.size(), 0);
         for (const tlg::PolyNode& l : prule.lines) t->hexline_plane = std::max(t->hexline_plane, of_plane[l.plane] += l.count);
         t->poly_planes = (uint32_t)align16(pstarts.size() * 4);
@@ -1890,7 +1906,7 @@ tlg_status eval_dispatch(const tlg_tables* t, const tlg_block* b, const tlg_outp
     tlg_status st = t->df ? eval_dfpoly(t, b, o, mask, ran, s, &found) : eval_poly(t, b, o, mask, ran, s, &found);
     if (found) return st;
   }
-  if (t->hexline_bytes > 0 && (is_auto || strategy == TLG_STRATEGY_DIRECT)) {
+  if (t->hexline_bytes > 0 && (is_auto || strategy == TLG_STRATEGY_DIRECT) && hexline_preferred(t, b, o, mask)) {
     bool found = false;
     tlg_status st = eval_hexline(t, b, o, mask, s, &found);
     if (found) return st;

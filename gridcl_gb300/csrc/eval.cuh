@@ -29,7 +29,8 @@
 //    triangles; the other f64 elements at few points or for points alone, else the polynomial kernel of
 //    eval_poly.cuh).
 //  - eval_loops_kernel<F, TD, GD>: K and the tile at run time (every other element and tile).
-// Hexahedra on f32 meshes and in split precision run the line kernel of eval_hexline.cuh.
+// Hexahedra on f32 meshes and in split precision run the line kernel of eval_hexline.cuh where
+// hexline_preferred takes it.
 #pragma once
 
 #include <cstdint>

@@ -85,3 +85,30 @@ def test_double_float_at_scattered_points(cuda, cell, degree, npts):
             a, b = got[f].to_host_cell_major(), want[f].to_host_cell_major()
             assert np.abs(a - b).max() <= 3e-13 * np.abs(b).max(), f
     assert ms(g, ps, ALL, "df64") <= 0.8 * ms(g, ps, ALL, "native")
+
+
+@pytest.mark.parametrize("precision", ["f32", "split"])
+@pytest.mark.parametrize("degree", [1, 2])
+def test_hexahedra_in_f32_and_split(cuda, degree, precision):
+    """The paired kernel's calls (bit for bit the loops kernel's values): points that share no line, few points,
+    points alone, and Q1 with a cell measure, whose sums it forms as it goes. The rest runs the line kernel."""
+    g = tg.Geometry.from_host(meshes.curved_box("Hexahedron", 22, degree, jitter=0.001),  # above 64 cells per SM
+                              dtype=torch.float32 if precision == "f32" else torch.float64)
+    mode = "native" if precision == "f32" else precision
+    cells = g.blocks[0].num_cells
+
+    def both(pts, names, measure=False):
+        ps = tg.PointSet("Hexahedron", pts, np.full(len(pts), 1.0 / len(pts)))
+        res = []
+        for strategy in ("auto", "loops"):
+            cm = torch.zeros(cells, dtype=torch.float32, device="cuda") if measure else None
+            with tg.with_strategy(strategy):
+                r = tg.geometric_factors_block(g, 0, ps, names, precision=mode, cell_measure=cm)
+            res.append([r[f].to_host_cell_major() for f in names] + ([cm.cpu().numpy()] if measure else []))
+        return all(np.array_equal(a, b) for a, b in zip(*res))
+
+    rule = tg.refcell.collapsed_rule("Hexahedron", (3, 3, 3))[0]
+    scattered = np.random.default_rng(3).uniform(0.05, 0.95, size=(27, 3))
+    assert both(scattered, ALL) and both(rule[:4], ALL) and both(rule, ("points",))
+    assert both(rule, ALL, measure=True) == (degree == 1)
+    assert not both(rule, ALL)
