@@ -9,9 +9,12 @@ namespace tlg {
 template <bool FN>
 static cudaError_t launch_sf_df(int td, int gd, int n, const SfArgs& a, size_t smem, cudaStream_t s, bool* found) {
   *found = true;
-  if (a.prism) {  // one step per CTA: P2 at 21 points, 300,000 cells, 0.595 ms persistent, 0.533 so
-    if (n == 2) return launch_persistent(sumfact_prism_df_kernel<2, FN>, a, a.padded, smem, s, true);
-    if (n == 3) return launch_persistent(sumfact_prism_df_kernel<3, FN>, a, a.padded, smem, s, true);
+  if (a.prism) {
+    // One step per CTA: P2 at 21 points, 300,000 cells, 0.595 ms persistent, 0.533 so; but det J alone, 128,000
+    // cells, 0.104 / 0.109, points alone 0.111 / 0.116 (P3 even).
+    const bool step = (a.mask & (kOutJacobian | kOutPinv | kOutFacetNormals)) != 0;
+    if (n == 2) return launch_persistent(sumfact_prism_df_kernel<2, FN>, a, a.padded, smem, s, step);
+    if (n == 3) return launch_persistent(sumfact_prism_df_kernel<3, FN>, a, a.padded, smem, s, step);
     if (n == 4) return launch_persistent(sumfact_prism_df_kernel<4, FN>, a, a.padded, smem, s, true);
     *found = false;
     return cudaSuccess;
