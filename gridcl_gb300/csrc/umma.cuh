@@ -63,6 +63,8 @@ struct UmmaArgs {
   // Work items: each tile's chunks in `groups` groups of `per_group` (the last ones padded with
   // zero tables; the table section holds chunks + kUmmaMaxGroups - 1 chunks).
   int groups, per_group;
+  // The rows kernel (umma_rows.cuh) cuts its runs at multiples of `unit` chunks: 1, or a tile's.
+  int unit;
 };
 
 constexpr int kUmmaMaxGroups = 8;

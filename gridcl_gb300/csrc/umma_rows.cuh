@@ -150,10 +150,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const __grid
   const bool issue_copies = !(a.err && a.err[2] == 1);
   const NT* nodes = static_cast<const NT*>(a.nodes);
   const uint32_t mask = a.mask;
-  // The (tile, chunk) pairs in tile order are cut into equal runs, one per CTA; an item is a run's part of
-  // one tile.
-  const int64_t pairs = (a.padded + kRowsCells - 1) / kRowsCells * a.chunks;
-  const int64_t first = pairs * blockIdx.x / gridDim.x, last = pairs * (blockIdx.x + 1) / gridDim.x;
+  // The (tile, chunk) pairs in tile order are cut into equal runs of units, one per CTA; an item is a run's
+  // part of one tile.
+  const int64_t units = (a.padded + kRowsCells - 1) / kRowsCells * a.chunks / a.unit;
+  const int64_t first = units * blockIdx.x / gridDim.x * a.unit, last = units * (blockIdx.x + 1) / gridDim.x * a.unit;
   const int run = (int)(last - first);
   const bool issuer = __shfl_sync(0xFFFFFFFFu, warp, 0) == kEpi;  // the issuing warp
 
