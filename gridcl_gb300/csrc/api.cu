@@ -2118,6 +2118,18 @@ tlg_status vjp_sumfact(const tlg_tables* t, const tlg::VjpArgs& v, cudaStream_t 
   return ok();
 }
 
+// Whether the f64 adjoint runs the polynomial kernel where the node-row kernel is compiled too: not at one point
+// (two on P3 tetrahedra) of a block that fills the device, whose coefficients and transposes one point does not
+// pay back. GB300, forward and adjoint with the node sums, ms, node rows / polynomial: one point, 280,000 P3
+// tetrahedra 0.75 / 1.17 (two points 1.22 / 1.37), P2 0.51 / 0.56, 140,608 Q2 hexahedra 0.43 / 0.53, 128,000 P2 prisms
+// 0.32 / 0.37, 320,000 P2 triangles 0.185 / 0.203.
+bool vjp_poly_preferred(const tlg_tables* t, const tlg_block* b) {
+  const bool rows = t->cell == tlg::kTetrahedron || t->cell == tlg::kPrism || t->cell == tlg::kHexahedron ||
+                    t->cell == tlg::kTriangle;
+  const bool p3 = t->cell == tlg::kTetrahedron && t->degree == 3;
+  return !rows || !(p3 ? t->q <= 2 : t->degree == 2 && t->q == 1) || b->num_cells < (int64_t)64 * 152;
+}
+
 // The f64 polynomial adjoint from the arguments of the node-row kernel; `found` is false where none
 // is compiled for the tables.
 tlg_status vjp_poly(const tlg_tables* t, const tlg_block* b, const tlg::VjpArgs& v, int family, cudaStream_t s,
@@ -2355,7 +2367,7 @@ tlg_status tlg_vjp_block(const tlg_tables* t, const tlg_block* b, const tlg_outp
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool sumfact = strategy == TLG_STRATEGY_SUMFACT || strategy == TLG_STRATEGY_AUTO;
   // f64 cells with a polynomial kernel: it takes the place of both.
-  if (t->poly_bytes > 0) {
+  if (t->poly_bytes > 0 && vjp_poly_preferred(t, b)) {
     const int family = sumfact && vjp_sumfact_preferred(t) ? TLG_STRATEGY_SUMFACT : TLG_STRATEGY_DIRECT;
     tlg_status st = vjp_poly(t, b, a, family, s, &found);
     if (found) return st;

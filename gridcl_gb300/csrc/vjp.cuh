@@ -24,8 +24,8 @@
 // The eight cells of a warp are consecutive: their contributions are staged in shared memory
 // and written as one contiguous run.
 //
-// What reaches it: split precision, and in f64 pyramids and P4 triangles (the other f64 cells run
-// the polynomial adjoint of vjp_poly.cuh).
+// What reaches it: split precision, and in f64 pyramids, P4 triangles and one-point rules (vjp_poly_preferred; the
+// other f64 cells run the polynomial adjoint of vjp_poly.cuh).
 //
 // SPLIT: f64 nodes shifted by node 0 in f64, FP32 arithmetic on two points at a time (FFMA2,
 // FMUL2 and FADD2 over the pair (q, q + 1)), f32 cotangents, contributions and fields.

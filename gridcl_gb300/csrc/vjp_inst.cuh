@@ -18,18 +18,19 @@ cudaError_t TLG_VJP_LAUNCH(int d, int k, const VjpArgs& a, size_t smem, cudaStre
   }
 #if TLG_VJP_SPLIT  // (f64: the polynomial kernel of vjp_poly.cuh)
   TLG_VJP(3, 4)
-  TLG_VJP(3, 10)
-  TLG_VJP(3, 20)
   TLG_VJP(3, 8)
-  TLG_VJP(3, 27)
   TLG_VJP(3, 6)
-  TLG_VJP(3, 18)
   TLG_VJP(2, 3)
-  TLG_VJP(2, 6)
   TLG_VJP(2, 10)
   TLG_VJP(2, 4)
   TLG_VJP(2, 9)
 #endif
+  // (f64: the one-point rules that vjp_poly_preferred leaves)
+  TLG_VJP(3, 10)
+  TLG_VJP(3, 20)
+  TLG_VJP(3, 27)
+  TLG_VJP(3, 18)
+  TLG_VJP(2, 6)
   TLG_VJP(3, 5)
   TLG_VJP(3, 14)
   TLG_VJP(3, 30)
