@@ -17,7 +17,11 @@
 // intrinsic (no compiler contraction), written once for scalars and for f32 pairs, so the sums
 // (x, J, and det J and K of volume cells) have the same bits for the same point whichever of the
 // kernels below runs. Surfaces differ in the last bits: the paired kernel forms their area
-// element, normal and K from one reciprocal square root (SurfacePair).
+// element, normal and K from one reciprocal square root (SurfacePair), the loops kernel at other tiles does
+// not. So do the polynomial and line kernels (eval_poly.cuh, eval_dfpoly.cuh, eval_hexline.cuh) from those
+// below: a call's bits depend on whether it asks for facet normals (double-float volume cells, hexahedra on f32
+// meshes and in split precision), on its rule, and on blocks above 64 cells per SM on the factors asked for
+// (poly_preferred, dfpoly_preferred, hexline_preferred).
 //
 // Kernels:
 //  - eval_pair_kernel<SPLIT, TD, GD, K>: f32 arithmetic on two quadrature points at once with
@@ -503,7 +507,9 @@ __device__ __noinline__ void recompute_f64(const double* __restrict__ nodes, con
 // 1,048,583 cells, split
 // precision, 0.462 -> 0.373 ms (527 -> 400 instructions per pair). Here len takes one Newton step on s y (s = |n|^2, y = rsqrt(s)) and each
 // quotient one residual step, which leaves them within an ulp, mostly correctly rounded. Pairs with an s
-// that is zero, subnormal, infinite or NaN take the operations of Factors.
+// outside [1.2e-30, 1e38] take the operations of Factors: the residuals s - g g and 1 - len y are exact as long as
+// the products' last bits (2^-48 of s) stay above the smallest subnormal, and 1 / s leaves the normal range above. s is
+// the fourth power of a length: edges below about 3e-8 or above 3e9 take that path throughout.
 struct SurfacePair {
   using A = Ar<float2>;
   float2 n[3], s2, len, inv;

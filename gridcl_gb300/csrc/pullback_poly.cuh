@@ -19,8 +19,8 @@
 //
 // Bound by the FP64 pipe (native f64, and the residuals of mixed precision): about 115 FP64
 // operations an iteration on a P2 tetrahedron. GB300, 48,000 P2 tetrahedra with 24 points, f64:
-// 20.9 -> 1.37 ms (generic kernel -> this one); 35,937 Q2 hexahedra with 27 points, mixed: 9.07 ->
-// 0.61 ms.
+// 20.9 -> 1.26 ms (generic kernel -> this one; 1.37 with the comparisons of newton_update on the FP64 pipe);
+// 35,937 Q2 hexahedra with 27 points, mixed: 9.07 -> 0.57 ms.
 #pragma once
 
 #include <algorithm>

@@ -1,6 +1,7 @@
 // Blackwell tensor-core evaluation (tcgen05) for volume cells of many nodes: the node-by-basis
 // contraction X^T Phi as a UMMA with FP32 accumulators in tensor memory. The policy runs it for cells of
-// 65 to 88 nodes (64 in split precision); those of 28 to 64 nodes run the kernel of umma_rows.cuh.
+// 65 to 88 nodes on f32 meshes and of 57 to 88 in split precision, whose heads and tails for 128 cells do not
+// fit shared memory (umma_rows_smem_bytes); those of 28 nodes on run the kernel of umma_rows.cuh.
 //
 // Per tile of 64 cells, for each coordinate g the A operand (M = 128 rows, K = nodes) holds the
 // TF32 heads of the cells' coordinates relative to their first node in rows 0-63 and the TF32

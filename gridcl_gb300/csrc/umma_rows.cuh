@@ -13,7 +13,7 @@
 // Bound: every partial product of a cell lands in the lane that stores the cell, so the epilogue (one
 // thread per cell, eight warps of four points a chunk) needs no exchange and no CTA-wide barrier. Warps
 // wait for a chunk's accumulators (mbarrier), load them, release the buffer (mbarrier, one arrival per
-// warp) and finish their points; a seventeenth warp issues the table copies and the MMAs, a chunk
+// warp) and finish their points; a ninth warp issues the table copies and the MMAs, a chunk
 // ahead of the epilogue. N = 64 because the MMAs of this shape are bound by reading A (66 cycles for
 // 128 x 32 x 8, counted on the 32-column kernel): one pass over A serves both halves of B.
 // The kernel of umma.cuh (heads in rows 0-63, tails in rows 64-127, summed over two warps through
