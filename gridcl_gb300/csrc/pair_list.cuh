@@ -6,7 +6,7 @@
 namespace tlg {
 
 // One step per CTA (launch_persistent): volume cells on f32 meshes where J is wanted and a cell stores at least
-// 170 values (P3 with det J alone: 18 points), so that its start and the CTA's table copy are small beside the
+// 120 values (18 nodes and more with det J alone: 18 points), so that its start and the CTA's table copy are small beside the
 // rest; and in split precision from P2 on where the FP64 subtractions (3 K per cell) are at most 6 % of the
 // values stored. GB300, ms, persistent / one step:
 // split P2 tetrahedra 24 points 1,572,864 cells 0.640 / 0.539 (5.7 %), 27 points 440,000 0.204 / 0.183, 64 points
@@ -14,7 +14,8 @@ namespace tlg {
 // (9 %); P1 tetrahedra 8 points 1,000,000 0.138 / 0.144; f32 P1 tetrahedra 8 points 1,500,000 0.193 / 0.164, P2
 // 24 points 1,000,000 0.388 / 0.329, P3 64 points 150,000 0.166 / 0.145, P2 prisms 27 points 0.141 / 0.126, P3 27
 // points det J alone 280,000 0.075 / 0.069; but of 280,000 f32 cells P1 8 points det J alone 0.0108 / 0.0123, points
-// alone 0.0085 / 0.0104, det J and K 0.0202 / 0.0213, P2 4 points four factors 0.0249 / 0.0269, P3 125 points alone
+// alone 0.0085 / 0.0104, det J and K 0.0202 / 0.0213 (6 points four factors, 1,500,000 cells: 0.143 / 0.125), P2 4
+// points four factors 0.0249 / 0.0269, P3 125 points alone
 // 0.167 / 0.180; f32 P2 triangles 9 points 800,000 0.049 / 0.053 and split P2 triangles 0.128 / 0.131.
 inline bool pair_one_step(bool split, int td, int k, const PairArgs& a) {
   if (td != 3) return false;
@@ -23,7 +24,7 @@ inline bool pair_one_step(bool split, int td, int k, const PairArgs& a) {
   for (int i = 0; i < 6; ++i)
     if ((a.mask >> i) & 1u) values += (int64_t)a.num_points * len[i];
   if (!split)
-    return (a.mask & ~(uint32_t)(kOutPoints | kOutCellMeasure)) && (values >= 170 || (k >= 20 && a.num_points >= 18));
+    return (a.mask & ~(uint32_t)(kOutPoints | kOutCellMeasure)) && (values >= 120 || (k >= 18 && a.num_points >= 18));
   return k >= 10 && 3 * k * 100 <= 6 * values;
 }
 
