@@ -839,7 +839,7 @@ def extra_p1_box():
 # What binds each mode's kernel, from its ncu capture (the profiles of the P2 tetrahedra): the
 # double-float and FP64 kernels are bound by an arithmetic pipe, not by HBM.
 BINDING = {
-    "df64": "issue 47 % over three pipes: FP64 39 %, ALU 38 %, FMA 32 % of active cycles (ncu, 32^3 x 6 case)",
+    "df64": "issue 46 % over three pipes: FP64 40 %, FMA 34 %, ALU 32 % of active cycles (ncu, 32^3 x 6 case)",
     "f64": "FP64 pipe: 91.0 % of active cycles (ncu)",
     "split": "HBM: stores of the f32 fields (ncu traffic 0.98 x the algorithmic bytes)",
     "f32": "HBM: stores of the f32 fields",

@@ -24,9 +24,9 @@
 // curved cells 8 %.
 //
 // Bound by the issue slots (50 % of them used at 16 warps per SM: dependent double-float chains, and 80-90 %
-// hits in the instruction cache) with the FP64 pipe 38 % and the integer pipe 37 % active. GB300, x, J, det J
+// hits in the instruction cache) with the FP64 pipe 40 % and the integer pipe 32 % active. GB300, x, J, det J
 // and K, ms, the former kernels (one thread or three lanes per cell) -> this one: P2 tetrahedra, 1,572,864
-// cells at 24 points 3.04 -> 1.91; Q2 hexahedra, 500,000 at 27 points 1.74 -> 1.38; P3 tetrahedra, 180,000 at
+// cells at 24 points 3.04 -> 1.91; Q2 hexahedra, 500,000 at 27 points 1.74 -> 1.36; P3 tetrahedra, 180,000 at
 // 64 points 2.36 -> 0.88; 1,000 P2 tetrahedra at 27 points 0.073 -> 0.032 (the host's call).
 #pragma once
 

@@ -201,8 +201,8 @@ tlg_status tlg_batch_destroy(tlg_batch* batch);
  * apply to its tables (the policy, direct, sumfact, cooperative, tensor; none when the caller has
  * set a strategy: an override on this thread or TLG_GEOM_STRATEGY), keeps the fastest (a forced
  * strategy replaces the policy only when more than 3 % faster), then candidate persistent grids
- * (0 and 1..8 CTAs per SM) for it (a grid replaces the occupancy limit only when more than 1 %
- * faster), and caches the choice per launch shape for the process; then, timing the
+ * (0 and 1..8 CTAs per SM; none where the block's kernel has a CTA per group of cells) for it (a grid
+ * replaces the occupancy limit only when more than 1 % faster), and caches the choice per launch shape for the process; then, timing the
  * whole graph as it runs in use (the median over 5 rounds of the mean of 4 back-to-back
  * launches), takes parallel branches over a serial chain only when more than 3 % faster in the
  * median and in the slowest round, runs one round of coordinate descent over each block's candidates
@@ -275,7 +275,8 @@ tlg_status tlg_vjp_block(const tlg_tables* tables, const tlg_block* block, const
  * outputs->pinv (det J and K of the range, tiled as tlg_eval_block writes them) are read instead
  * of recomputed, the other output pointers are ignored. Volume cells (TD = GD = 3), f64 or
  * split-precision tables: hexahedra Q1/Q2 at tensor-product rules by the sum-factorised
- * transposed contraction (rows as tlg_vjp_block's sum-factorised adjoint, bit for bit), other
+ * transposed contraction (in split precision tlg_vjp_block's rows bit for bit; in f64 to rounding, where
+ * that runs the polynomial adjoint), other
  * cells and rules from the tables' node rows where they and 12 * 16 values per point fit in
  * shared memory; TLG_ERR_UNSUPPORTED otherwise. A forward pass plus this adjoint moves more bytes
  * than the fused pass but needs neither the coordinates nor the forward contraction here. No
