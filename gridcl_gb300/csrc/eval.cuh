@@ -20,8 +20,8 @@
 // element, normal and K from one reciprocal square root (SurfacePair), the loops kernel at other tiles does
 // not. So do the polynomial and line kernels (eval_poly.cuh, eval_dfpoly.cuh, eval_hexline.cuh) from those
 // below: a call's bits depend on whether it asks for facet normals (double-float volume cells, hexahedra on f32
-// meshes and in split precision), on its rule, and on blocks above 64 cells per SM on the factors asked for
-// (poly_preferred, dfpoly_preferred, hexline_preferred).
+// meshes and in split precision), on its rule, and on the factors asked for (double-float; the others on
+// blocks of 64 cells per SM and more): poly_preferred, dfpoly_preferred, hexline_preferred.
 //
 // Kernels:
 //  - eval_pair_kernel<SPLIT, TD, GD, K>: f32 arithmetic on two quadrature points at once with
