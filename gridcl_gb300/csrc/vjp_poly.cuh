@@ -237,6 +237,18 @@ __global__ void __launch_bounds__(192, 2) vjp_poly_kernel(const __grid_constant_
 #pragma unroll
                 for (int g = 0; g < GD; ++g) jb[d * GD + g] = __dmul_rn(s, kk[g * TD + d]);
             }
+            // A cotangent that is not finite reaches every node of the cell, as through the Lagrange functions (0
+            // times NaN), also from a middle point, whose low coefficients only some nodes are in: the highest
+            // coefficient is in every node's row.
+            if constexpr (TENSOR && N == 3) {
+#pragma unroll
+              for (int g = 0; g < GD; ++g) {
+                bool bad = has_x && poly_bad(xb[g]);
+#pragma unroll
+                for (int d = 0; d < TD; ++d) bad = bad || poly_bad(jb[d * GD + g]);
+                if (bad) cb[((K - 1) * GD + g) * W + lane] = poly_nan();
+              }
+            }
             if (MID && x.mid) poly_point_bar<CELL, P, MID>(x, has_x, xb, jb, Ab, Db, Eb);
             else poly_point_bar<CELL, P, false>(x, has_x, xb, jb, Ab, Db, Eb);
           }
